@@ -95,12 +95,19 @@ struct WarpBulk {
   // Stage matrix A (n x n complex128, row stride lda) into M (row stride lds).
   // Warp-uniform result: false if the wait ran out (M is then not valid).
   __device__ bool load(const double2 *A, int n, int lda, double2 *M, int lds, int lane) {
+    return load_rows(A, n, n, lda, M, lds, n, lane);
+  }
+  // Stage `rows` consecutive rows of n entries (of consecutive n-row matrices)
+  // into M, n rows of a matrix every mrows rows of M.
+  __device__ bool load_rows(const double2 *A, int rows, int n, int lda, double2 *M, int lds,
+                            int mrows, int lane) {
     __syncwarp();
     fence_proxy_async_smem();
-    if (lane == 0) mbar_arrive_expect_tx(bar, (unsigned)(n * n * 16));
+    if (lane == 0) mbar_arrive_expect_tx(bar, (unsigned)(rows * n * 16));
     __syncwarp();
-    for (int i = lane; i < n; i += 32)
-      bulk_g2s(M + i * lds, A + (size_t)i * lda, (unsigned)(n * 16), bar);
+    for (int i = lane; i < rows; i += 32)
+      bulk_g2s(M + (mrows == n ? i : i + i / n * (mrows - n)) * lds, A + (size_t)i * lda,
+               (unsigned)(n * 16), bar);
     bool ok = mbar_wait(bar, phase, kBulkWaitTries);
     ok = __all_sync(kFull, ok);
     if (!ok) {
@@ -113,10 +120,14 @@ struct WarpBulk {
   }
 };
 
+// L2 prefetch of `rows` rows of n complex128 entries with row stride lda.
+__device__ __forceinline__ void prefetch_rows_l2(const double2 *A, int rows, int n, int lda) {
+  prefetch_l2_bulk(A, (unsigned)(((size_t)(rows - 1) * lda + n) * 16));
+}
 // L2 prefetch of an n x n complex128 matrix with row stride lda (the span
 // from its first entry to the end of its last row).
 __device__ __forceinline__ void prefetch_matrix_l2(const double2 *A, int n, int lda) {
-  prefetch_l2_bulk(A, (unsigned)(((size_t)(n - 1) * lda + n) * 16));
+  prefetch_rows_l2(A, n, n, lda);
 }
 
 }  // namespace lufqhe

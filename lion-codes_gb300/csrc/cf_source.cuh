@@ -145,6 +145,12 @@ struct CfSource {
   }
 };
 
+__device__ __forceinline__ void load_rows(const CfSource &s, long long b0, int rows, int n,
+                                          double2 *M, int lds, int mrows, int lane) {
+  for (int q = lane; q < rows; q += 32)
+    s.row(b0 + q / n, n, q % n, M + (q + q / n * (mrows - n)) * lds);
+}
+
 // Rows for the extended-precision correction (fp64_correct.cuh), which
 // re-reads the matrix it corrects.
 struct CfRow {

@@ -208,6 +208,44 @@ struct LllSource {
   }
 };
 
+// `rows` consecutive rows of a batch (row q is row q % n of matrix b0 + q / n)
+// into M at row stride lds, n rows of a matrix every mrows rows of M, by one
+// warp. No finiteness check: for kernels that look at every entry anyway.
+template <class T>
+__device__ __forceinline__ double2 load_entry(const T *p);
+template <>
+__device__ __forceinline__ double2 load_entry<double2>(const double2 *p) {
+  return __ldg(p);
+}
+template <>
+__device__ __forceinline__ double2 load_entry<float2>(const float2 *p) {
+  return Dense32Source::widen(__ldg(p));
+}
+template <class T>
+__device__ __forceinline__ void load_rows_dense(const T *A, int lda, int rows, int n, double2 *M,
+                                                int lds, int mrows, int lane) {
+  BlockWalk w(lane, n);
+#pragma unroll 4
+  for (int e = lane; e < rows * n; e += 32) {
+    const int q = mrows == n ? w.i : w.i + w.i / n * (mrows - n);
+    M[q * lds + w.k] = load_entry(A + (size_t)w.i * lda + w.k);
+    w.next(n);
+  }
+}
+__device__ __forceinline__ void load_rows(const DenseSource &s, long long b0, int rows, int n,
+                                          double2 *M, int lds, int mrows, int lane) {
+  load_rows_dense(s.A + (size_t)b0 * n * s.lda, s.lda, rows, n, M, lds, mrows, lane);
+}
+__device__ __forceinline__ void load_rows(const Dense32Source &s, long long b0, int rows, int n,
+                                          double2 *M, int lds, int mrows, int lane) {
+  load_rows_dense(s.A + (size_t)b0 * n * s.lda, s.lda, rows, n, M, lds, mrows, lane);
+}
+__device__ __forceinline__ void load_rows(const LllSource &s, long long b0, int rows, int n,
+                                          double2 *M, int lds, int mrows, int lane) {
+  for (int q = lane; q < rows; q += 32)
+    lll_row_rn(__ldg(s.Z + (size_t)b0 * n + q), n, M + (q + q / n * (mrows - n)) * lds);
+}
+
 // RN(a / b) for b > 0 given y = RN(1/b): Markstein's correction (P. Markstein,
 // IBM J. Res. Dev. 34(1), 1990): q0 = RN(a*y) is refined once to a faithful
 // q1, then q2 = RN(q1 + RN(a - b*q1)*y) is the correctly rounded quotient when

@@ -39,12 +39,12 @@ float g_mixed_theta = 0.1f;
 int g_mixed_refine = 1;
 
 // Device memory a batched mixed call takes from the library's pool while it
-// runs, its state block (CallState): the head, for n >= 24 the pending list
+// runs, its state block (CallState): the head, for n >= 17 the pending list
 // (one entry per matrix) and, for n = 24 and 32, the saved matrices.
 size_t mixed_workspace_bytes(int n, long long batch) {
   if (fp64_share_64k(n) >= 65536u || batch == 0) return 0;
   auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
-  if (n < kDeferMinN) return kHeadBytes;  // at most the work counter
+  if (n <= 16) return kHeadBytes;  // at most the work counter
   size_t bytes = kHeadBytes + up((size_t)batch * sizeof(unsigned int));
   if (g_mixed_refine && (n == 24 || n == 32)) {
     long long cap = std::max<long long>(256, (long long)(kRefineShare * (double)batch));

@@ -469,6 +469,24 @@ __device__ bool mixed_factor(const MixedSmem &S, int n, int lane, float theta2, 
   return mixed_finish<2>(S.Af, R, n, lds, lane, theta2, exp_sum, prod, corr);
 }
 
+// log|det| and phase from the float-float diagonal product, its exponent, the
+// correction and the parity. Out of line: it runs once per 32 matrices, and its
+// FP64 log and atan2 (700 instructions a copy) are better kept out of the hot
+// loops, which are larger than the instruction cache as it is.
+struct LogPolar {
+  double la, ph;
+};
+__device__ __noinline__ LogPolar finish_log_polar(float xh, float xl, float yh, float yl, int e,
+                                                  float cx, float cy, int par) {
+  const double re = __dadd_rn((double)xh, (double)xl);
+  const double im = __dadd_rn((double)yh, (double)yl);
+  const double m2 = __fma_rn(re, re, __dmul_rn(im, im));
+  LogPolar r;
+  r.la = __dadd_rn(__fma_rn((double)e, kLn2, __dmul_rn(0.5, log(m2))), (double)cx);
+  r.ph = wrap_phase(__dadd_rn(__dadd_rn(atan2(im, re), (double)cy), par ? kPi : 0.0));
+  return r;
+}
+
 // Deferred FP64 finalisation: lane L holds the L-th accepted matrix of the
 // current group of 32; one warp-wide log/atan2 then serves all 32.
 struct DeferredOut {
@@ -481,14 +499,10 @@ struct DeferredOut {
   __device__ __forceinline__ void flush(int lane, double *logabs, double *phase, int8_t *parity,
                                         int32_t *status) {
     if (lane < cnt && slot_b >= 0) {
-      const double re = __dadd_rn((double)slot_p.xh, (double)slot_p.xl);
-      const double im = __dadd_rn((double)slot_p.yh, (double)slot_p.yl);
-      const double m2 = __fma_rn(re, re, __dmul_rn(im, im));
-      const double la =
-          __dadd_rn(__fma_rn((double)slot_e, kLn2, __dmul_rn(0.5, log(m2))), (double)slot_c.x);
-      const double ph = __dadd_rn(__dadd_rn(atan2(im, re), (double)slot_c.y), slot_par ? kPi : 0.0);
-      logabs[slot_b] = la;
-      if (phase) phase[slot_b] = wrap_phase(ph);
+      const LogPolar r = finish_log_polar(slot_p.xh, slot_p.xl, slot_p.yh, slot_p.yl, slot_e,
+                                          slot_c.x, slot_c.y, slot_par);
+      logabs[slot_b] = r.la;
+      if (phase) phase[slot_b] = r.ph;
       if (parity) parity[slot_b] = (int8_t)slot_par;
       if (status) status[slot_b] = 0;
     }

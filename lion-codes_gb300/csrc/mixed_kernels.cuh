@@ -37,10 +37,12 @@
 // the index of a rejected matrix to the call's pending list; the second
 // kernel deals the list's entries out to its warps at a fixed stride for FP64
 // while the other warps refine the saved matrices, so the FP64 and FP32 pipes
-// work side by side. For n < 24 the FP64 refactorisations are cheap and rare enough that
-// the second launch costs more than it saves; there the FP32 pass refines and
-// refactorises in place, and so does the n >= 24 variant that reads its batch
-// over the host link (INPLACE). The kernels take their matrices from a source:
+// work side by side. The other sizes take the lane-grid path (mixed_grid.cuh): for
+// n <= 16, where the FP64 refactorisations are cheap and rare enough that a
+// second launch costs more than it saves, it refines and refactorises in place,
+// and so does the n = 24, 32 variant that reads its batch over the host link
+// (INPLACE); at 17 <= n <= 31 (without a register-tiled kernel) the rejected
+// matrices go to lup_mixed_fallback_kernel. The kernels take their matrices from a source:
 // dense matrices in the reference layout, or lowest-Landau-level orbital
 // matrices built from particle coordinates.
 //
@@ -60,6 +62,7 @@
 
 #include "bulk_copy.cuh"
 #include "mixed_core.cuh"
+#include "mixed_grid.cuh"
 
 namespace lufqhe {
 
@@ -76,11 +79,10 @@ using namespace mixed;
 // Warps per CTA and CTAs per SM the register-tiled kernels are compiled for:
 // the register budget this leaves (65536 / (32 warps blocks)) is what lets the
 // SM hold that many warps, whichever of registers or shared memory binds.
-// n = 24: 3-warp CTAs, 5 per SM (15 KB of shared memory per warp); n <= 16:
-// 4-warp CTAs, 4 per SM; n = 32: shared memory allows 8 warps whatever the
-// registers.
+// n = 24: 3-warp CTAs, 5 per SM (15 KB of shared memory per warp); n = 32:
+// shared memory allows 8 warps whatever the registers.
 constexpr int tile_max_warps(int n) { return n == 24 ? 3 : 4; }
-constexpr int tile_min_ctas(int n) { return n == 24 ? 5 : n == 32 ? 1 : 4; }
+constexpr int tile_min_ctas(int n) { return n == 24 ? 5 : 1; }
 
 // Head of a call's state block (zeroed on the call's stream before the first
 // kernel). Behind it: the pending list of the FP64 pass (one entry per matrix
@@ -114,6 +116,10 @@ __device__ __forceinline__ long long claim_matrix(CallHead *head, int lane, long
 constexpr unsigned int kPendRouted = 0x80000000u;
 
 constexpr int kDeferMinN = 24;
+// The same of the lane-grid kernels: shared memory holds 16 warps an SM at
+// NP = 16 (13.5 KB each), 15 at 24 (14.8 KB) and 8 at 32 (25.7 KB).
+constexpr int grid_warps(int np) { return np == 24 ? 3 : 4; }
+constexpr int grid_min_ctas(int np) { return np == 24 ? 5 : np == 32 ? 2 : 4; }
 // Warps of the FP64 pass's CTA (one CTA per SM).
 constexpr int kFallbackMaxWarps = 20;
 // Warps of a CTA of the correction pass after the finish kernel.
@@ -246,6 +252,139 @@ __global__ void __launch_bounds__(kMaxWarpsMixed * 32)
 }
 
 
+// F of one matrix from the grid path's row stride to stride N + 1, in place.
+template <int NP, int N>
+__device__ __forceinline__ void repack_f(float2 *F, int lane) {
+  constexpr int K = (N * N + 31) / 32;
+  float2 v[K];
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < K; ++q) {
+    const int e = lane + 32 * q;
+    if (e < N * N) v[q] = F[e / N * (NP + 2) + e % N];
+  }
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < K; ++q) {
+    const int e = lane + 32 * q;
+    if (e < N * N) F[e / N * (N + 1) + e % N] = v[q];
+  }
+  __syncwarp();
+}
+
+// The FP32 pass of the lane-grid path: each warp takes Grid::G consecutive
+// matrices at a time. NC = n for the register-tiled sizes, 0 for the generic
+// rule. DEFER: rejected matrices go to the call's pending list; else they are
+// refined or refactorised in FP64 right away, one at a time by the whole warp.
+template <int NP, int LPM, int NC, bool DEFER, class Src>
+__global__ void __launch_bounds__(grid_warps(NP) * 32, grid_min_ctas(NP))
+    lup_mixed_grid_kernel(Src src, int n_rt, long long batch, float theta2,
+                          unsigned int share64k, CallHead *head, unsigned int *pend, int refine,
+                          int bulk, double *__restrict__ logabs, double *__restrict__ phase,
+                          int8_t *__restrict__ parity, int32_t *__restrict__ status) {
+  using Gd = Grid<NP, LPM>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr bool BULK = std::is_same<Src, DenseSource>::value;
+  const int n = NC ? NC : n_rt;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int grp = lane / LPM;
+  unsigned char *base = smem_raw + (size_t)warp * Gd::kWarpBytes;
+  float4 *HLw = reinterpret_cast<float4 *>(base);
+  float2 *Fw = reinterpret_cast<float2 *>(HLw + Gd::G * Gd::kHL);
+  int *Iw = reinterpret_cast<int *>(Fw + Gd::G * Gd::kF);
+  double2 *M = reinterpret_cast<double2 *>(HLw);
+  __shared__ __align__(8) uint64_t bars[grid_warps(NP)];
+  WarpBulk wb;
+  if constexpr (BULK)
+    if (bulk) wb.init(&bars[warp], lane);
+
+  DeferredOut out;
+  const long long units = (batch + Gd::G - 1) / Gd::G;
+  long long u = claim_matrix(head, lane, -1);
+  long long nu = u < units ? claim_matrix(head, lane, u) : units;
+  for (; u < units; u = nu, nu = u < units ? claim_matrix(head, lane, u) : units) {
+    const long long b0 = u * Gd::G;
+    const int cnt = (int)min((long long)Gd::G, batch - b0);
+    __syncwarp();
+    bool staged = false;
+    if constexpr (BULK) {
+      if (bulk && !wb.broken) {
+        if (nu < units && lane == 0) {
+          const int ncnt = (int)min((long long)Gd::G, batch - nu * Gd::G);
+          prefetch_rows_l2(src.A + (size_t)(nu * Gd::G) * n * src.lda, ncnt * n, n, src.lda);
+        }
+        if (!wb.load_rows(src.A + (size_t)b0 * n * src.lda, cnt * n, n, src.lda, M, Gd::LDH, NP,
+                          lane)) {
+          for (int q = 0; q < cnt; ++q)
+            emit_wait_timeout(lane, b0 + q, logabs, phase, parity, status);
+          continue;
+        }
+        staged = true;
+      }
+    }
+    if (!staged) load_rows(src, b0, cnt * n, n, M, Gd::LDH, NP, lane);
+    __syncwarp();
+    CFF prod;
+    int exp_sum, par;
+    float2 corr;
+    int code = grid_factor<NP, LPM, NC, !DEFER>(HLw + grp * Gd::kHL, Fw + grp * Gd::kF,
+                                                Iw + grp * 2 * NP, n, lane, theta2, prod, exp_sum,
+                                                corr, par);
+    bool routed = false;
+    if (share64k && grp < cnt && code != TILE_NONFINITE) {
+      routed = route_fp64_entry(src.first(b0 + grp, n), share64k);
+      if (routed) code = TILE_REJECT;
+    }
+#pragma unroll 1
+    for (int q = 0; q < cnt; ++q) {
+      const int from = q * LPM;
+      const int cq = __shfl_sync(kFull, code, from);
+      const CFF pq = shfl_cff(prod, from, false);
+      const int eq = __shfl_sync(kFull, exp_sum, from);
+      const int rq = __shfl_sync(kFull, par, from);
+      float2 kq = shfl2(corr, from);
+      const long long b = b0 + q;
+      if (cq == TILE_ACCEPT) {
+        out.push(lane, b, pq, eq, kq, rq, logabs, phase, parity, status);
+        continue;
+      }
+      if (cq == TILE_NONFINITE) {
+        emit_nonfinite(lane, b, logabs, phase, parity, status);
+        continue;
+      }
+      const bool rt = __shfl_sync(kFull, (int)routed, from) != 0;
+      if constexpr (DEFER) {
+        defer_fp64(head, pend, b, lane, rt);
+      } else {
+        float4 *HLq = HLw + q * Gd::kHL;
+        float2 *Fq = Fw + q * Gd::kF;
+        int *Iq = Iw + q * 2 * NP;
+        if constexpr (NC != 0) {
+          if (cq == TILE_REFINE && refine) {
+            float2 *Rm = reinterpret_cast<float2 *>(HLq);
+            repack_f<NP, NC>(Fq, lane);
+            if (mixed_refine_tile<NC>(Fq, Rm, Rm + NC * (NC + 1), reinterpret_cast<float2 *>(Iq),
+                                      lane, theta2, tile_la_est(pq, eq), kq)) {
+              out.push(lane, b, pq, eq, kq, rq, logabs, phase, parity, status);
+              continue;
+            }
+          }
+        }
+        // the matrix again in this group's area, its row scales after it where
+        // the padding leaves room (n < NP), else over F (sizes up to 16 have no
+        // correction, which would use F)
+        double *hold = n < NP ? reinterpret_cast<double *>(HLq + (size_t)n * (n + 1))
+                              : reinterpret_cast<double *>(Fq);
+        fallback_fp64_src(src, b, n, reinterpret_cast<double2 *>(HLq), n + 1, hold, lane, b,
+                          logabs, phase, parity, status,
+                          rt ? LUFQHE_ST_FP64 : LUFQHE_ST_FALLBACK);
+      }
+    }
+  }
+  out.flush(lane, logabs, phase, parity, status);
+}
+
+
 template <int N, class Src, bool INPLACE = false>
 __global__ void __launch_bounds__(tile_max_warps(N) * 32, tile_min_ctas(N))
     lup_mixed_tile_kernel(Src src, long long batch, float theta2,
@@ -256,11 +395,11 @@ __global__ void __launch_bounds__(tile_max_warps(N) * 32, tile_min_ctas(N))
                           double *__restrict__ phase, int8_t *__restrict__ parity,
                           int32_t *__restrict__ status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  // n >= 24: every FP64 factorisation goes to the FP64 pass, so this kernel
-  // carries no FP64 factorisation code (a smaller instruction footprint).
-  // INPLACE keeps them in this kernel: for a batch read over the host link,
-  // where the FP32 pass waits on the link and has compute to spare.
-  constexpr bool DEFER = !INPLACE && N >= kDeferMinN;
+  // every FP64 factorisation goes to the FP64 pass, so this kernel carries no
+  // FP64 factorisation code (a smaller instruction footprint). INPLACE keeps
+  // them in this kernel: for a batch read over the host link, where the FP32
+  // pass waits on the link and has compute to spare.
+  constexpr bool DEFER = !INPLACE;
   // complex128 device batches: the matrix is staged by bulk copies (bulk != 0)
   constexpr bool BULK = !INPLACE && std::is_same<Src, DenseSource>::value;
   constexpr int LDS = N + 1;
@@ -344,11 +483,11 @@ __global__ void __launch_bounds__(tile_max_warps(N) * 32, tile_min_ctas(N))
                                 reinterpret_cast<const float2 *>(HL), prod, exp_sum, par, lane)))
         defer_fp64(head, pend, b, lane, false);
     } else {
-      // in place: the refinement (refine_cap != 0), then FP64 (n < 24, where
-      // both are rare, and the host-link variant, which has compute to spare)
+      // in place: the refinement (refine_cap != 0), then FP64 (the host-link
+      // variant, which has compute to spare)
       const int code =
           mixed_factor_tile_ex<N, true>(HL, F, er, ec, lane, theta2, prod, exp_sum, corr, par);
-      if (code == TILE_NONFINITE) {  // a staged matrix (the others were checked on load)
+      if (code == TILE_NONFINITE) {
         emit_nonfinite(lane, b, logabs, phase, parity, status);
         continue;
       }
@@ -357,9 +496,9 @@ __global__ void __launch_bounds__(tile_max_warps(N) * 32, tile_min_ctas(N))
            mixed_refine_tile<N>(F, reinterpret_cast<float2 *>(HL),
                                 reinterpret_cast<float2 *>(HL) + N * (N + 1),
                                 reinterpret_cast<float2 *>(er), lane, theta2,
-                                tile_la_est(prod, exp_sum), corr)))
+                                tile_la_est(prod, exp_sum), corr))) {
         out.push(lane, b, prod, exp_sum, corr, par, logabs, phase, parity, status);
-      else if constexpr (INPLACE) {
+      } else {
         // the factors (and the warp's copy of the matrix) are listed for the
         // correction pass, so that no warp stops reading the link for one
         const FacList fl{&head->corr_count, corr_list, corr_cap, 1};
@@ -367,9 +506,6 @@ __global__ void __launch_bounds__(tile_max_warps(N) * 32, tile_min_ctas(N))
                                              logabs, phase, parity, status, LUFQHE_ST_FALLBACK,
                                              &cs, corr_list != nullptr ? &fl : nullptr);
       }
-      else
-        fallback_fp64_src(src, b, N, M, LDS, hold, lane, b, logabs, phase, parity, status,
-                          LUFQHE_ST_FALLBACK, &cs);
     }
   }
   out.flush(lane, logabs, phase, parity, status);
@@ -696,7 +832,7 @@ int launch_mixed_tile(Src src, long long batch, float theta2, double *logabs, do
   int grid = (int)(want < cap ? want : cap);
   // n >= 24 from device memory: the refinements and FP64 refactorisations go
   // to the finish kernel through the call's pending list and saved matrices
-  const bool two_pass = N >= kDeferMinN && !inplace;
+  const bool two_pass = !inplace;
   long long refine_cap = 0;
   size_t refine_bytes = 0;
   if (two_pass && g_mixed_refine) {
@@ -766,6 +902,59 @@ int launch_mixed_tile(Src src, long long batch, float theta2, double *logabs, do
   return cs.release(stream, rc);
 }
 
+template <int NP, int LPM, int NC, bool DEFER, class Src>
+int launch_mixed_grid(Src src, int n, long long batch, float theta2, double *logabs,
+                      double *phase, int8_t *parity, int32_t *status, cudaStream_t stream) {
+  using Gd = Grid<NP, LPM>;
+  auto kern = lup_mixed_grid_kernel<NP, LPM, NC, DEFER, Src>;
+  constexpr int warps = grid_warps(NP);
+  const size_t smem = Gd::kWarpBytes * warps;
+  int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)smem),
+                      "cudaFuncSetAttribute(mixed grid)");
+  if (rc) return rc;
+  int per_sm = 0;
+  rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, smem),
+                  "occupancy(mixed grid)");
+  if (rc) return rc;
+  if (per_sm < 1) per_sm = 1;
+  const long long units = (batch + Gd::G - 1) / Gd::G;
+  const long long want = (units + warps - 1) / warps;
+  const long long cap = (long long)device_sm_count() * per_sm;
+  const int grid = (int)(want < cap ? want : cap);
+  CallState cs;
+  if (DEFER || needs_counter(units, (long long)grid * warps)) {
+    rc = cs.acquire(DEFER ? (size_t)batch : 0, 0, 0, stream);
+    if (rc) return cs.release(stream, rc);
+  }
+  {
+    KernelTimer timer("lup_mixed_grid_kernel", n, stream);
+    kern<<<grid, warps * 32, smem, stream>>>(src, n, batch, theta2, fp64_share_64k(n), cs.head,
+                                             cs.pend, g_mixed_refine, bulk_for(src), logabs,
+                                             phase, parity, status);
+    timer.stop();
+  }
+  rc = check_cuda(cudaGetLastError(), "lup_mixed_grid_kernel launch");
+  if constexpr (DEFER)
+    if (!rc)
+      rc = launch_fallback(src, n, cs.head, cs.pend, batch, logabs, phase, parity, status, stream);
+  return cs.release(stream, rc);
+}
+
+// n <= 16: several matrices per warp, except in a batch of at most one matrix
+// per SM sub-partition, where a warp each has the least latency (64 LLL matrices
+// of n = 16: 23.2 us a call with two per warp, 18.7 us with one).
+template <int NP, int LPM, int NC, class Src>
+int launch_mixed_small(Src src, int n, long long batch, float theta2, double *logabs,
+                       double *phase, int8_t *parity, int32_t *status, cudaStream_t stream) {
+  constexpr int NP1 = NP == 12 ? 16 : NP;  // whole 8-column slots
+  if (batch <= 4ll * device_sm_count())
+    return launch_mixed_grid<NP1, 32, NC, false>(src, n, batch, theta2, logabs, phase, parity,
+                                                 status, stream);
+  return launch_mixed_grid<NP, LPM, NC, false>(src, n, batch, theta2, logabs, phase, parity,
+                                               status, stream);
+}
+
 // Sources whose matrices are always of odd order (CF matrices, n = 2Q + 3)
 // never reach the register-tiled kernels, which exist for even n only.
 template <class S, class = void>
@@ -786,15 +975,21 @@ int launch_mixed_src(Src src, int n, long long batch, double *logabs, double *ph
   const float th2 = g_mixed_theta * g_mixed_theta;
   if constexpr (has_even_n<Src>::value) {
     switch (n) {
-      case 6: return launch_mixed_tile<6>(src, batch, th2, logabs, phase, parity, status, stream, inplace);
-      case 8: return launch_mixed_tile<8>(src, batch, th2, logabs, phase, parity, status, stream, inplace);
-      case 12: return launch_mixed_tile<12>(src, batch, th2, logabs, phase, parity, status, stream, inplace);
-      case 16: return launch_mixed_tile<16>(src, batch, th2, logabs, phase, parity, status, stream, inplace);
+      case 6: return launch_mixed_small<8, 8, 6>(src, n, batch, th2, logabs, phase, parity, status, stream);
+      case 8: return launch_mixed_small<8, 8, 8>(src, n, batch, th2, logabs, phase, parity, status, stream);
+      case 12: return launch_mixed_small<12, 16, 12>(src, n, batch, th2, logabs, phase, parity, status, stream);
+      case 16: return launch_mixed_small<16, 16, 16>(src, n, batch, th2, logabs, phase, parity, status, stream);
       case 24: return launch_mixed_tile<24>(src, batch, th2, logabs, phase, parity, status, stream, inplace);
       case 32: return launch_mixed_tile<32>(src, batch, th2, logabs, phase, parity, status, stream, inplace);
       default: break;
     }
   }
+  // other sizes on the lane grid of the next size up
+  if (n <= 8) return launch_mixed_small<8, 8, 0>(src, n, batch, th2, logabs, phase, parity, status, stream);
+  if (n <= 12) return launch_mixed_small<12, 16, 0>(src, n, batch, th2, logabs, phase, parity, status, stream);
+  if (n <= 16) return launch_mixed_small<16, 16, 0>(src, n, batch, th2, logabs, phase, parity, status, stream);
+  if (n <= 24) return launch_mixed_grid<24, 32, 0, true>(src, n, batch, th2, logabs, phase, parity, status, stream);
+  if (n <= 32) return launch_mixed_grid<32, 32, 0, true>(src, n, batch, th2, logabs, phase, parity, status, stream);
   const size_t per_warp = mixed_smem_per_warp(n);
   const size_t optin = device_smem_optin();
   int warps = (int)(optin / per_warp);

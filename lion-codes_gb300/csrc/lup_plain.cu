@@ -1,11 +1,11 @@
 // Plain FP64 batched complex LUP determinant.
 //
-// One warp factorises one matrix at a time, looping over the batch with a
-// grid stride. The matrix sits in shared memory (row stride n+1 complex so a
-// column read by 32 lanes hits 32 different banks); the right-looking update
-// of the (n-1-j)^2 trailing block is spread over all 32 lanes, so the FP64
-// pipe runs with full lanes until the block is smaller than a warp. The
-// factorisation itself (pivot rule, arithmetic) lives in lup_fp64.cuh.
+// A warp factorises 1 to 8 matrices at a time (n <= 32, by size and batch; a
+// CTA takes one above), looping over the batch with a grid stride. The matrices
+// sit in shared memory (odd row stride, so a column read by a group of lanes
+// hits different banks); the right-looking update of each (n-1-j)^2 trailing
+// block is spread over the matrix's lanes. The factorisation itself (pivot
+// rule, arithmetic) lives in lup_fp64.cuh and lup_fp64_sub.cuh.
 // The determinant is returned in log-polar form: the reference multiplies the
 // diagonal directly (LU-fqhe/src/LUCoreCPU.cu:256-265), which overflows for
 // lowest-Landau-level matrices.
@@ -18,6 +18,7 @@
 #include "cf_source.cuh"
 #include "fp64_correct.cuh"
 #include "lup_fp64.cuh"
+#include "lup_fp64_sub.cuh"
 
 namespace lufqhe {
 
@@ -25,17 +26,15 @@ namespace {
 
 constexpr int kMaxWarpsPlain = 8;
 
-// Out: element type of the in-place factors (double2, or float2 for the
-// reference's complex64 buffers). CORRECT: the mixed mode's FP64 route for
-// 17 <= n <= 32 (this warp kernel's sizes), whose log-determinants get the
-// extended-precision correction (fp64_correct_warp; its scratch follows the
-// row scales in shared memory).
-template <int ARITH, class Src, class Out = double2, bool CORRECT = false>
+// The mixed mode's FP64 route for 17 <= n <= 32, where the policy sends a whole
+// batch there: one warp per matrix, whose log-determinant gets the
+// extended-precision correction (fp64_correct_warp; its scratch follows the row
+// scales in shared memory).
+template <class Src>
 __global__ void __launch_bounds__(kMaxWarpsPlain * 32)
-    lup_plain_kernel(Src src, Out *__restrict__ Aout, int n, int lda,
-                     long long batch, double *__restrict__ logabs, double *__restrict__ phase,
-                     int8_t *__restrict__ parity, int32_t *__restrict__ status,
-                     int status_or, int bulk) {
+    lup_plain_correct_kernel(Src src, int n, long long batch, double *__restrict__ logabs,
+                             double *__restrict__ phase, int8_t *__restrict__ parity,
+                             int32_t *__restrict__ status, int status_or, int bulk) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warps = blockDim.x >> 5;
   const int warp = threadIdx.x >> 5;
@@ -45,13 +44,10 @@ __global__ void __launch_bounds__(kMaxWarpsPlain * 32)
   double *hold_all = reinterpret_cast<double *>(reinterpret_cast<double2 *>(smem_raw) +
                                                 (size_t)warps * n * lds);
   double *hold = hold_all + warp * 2 * n;
-  CorrScratch cs{};
-  if constexpr (CORRECT) {
-    float2 *F_all = reinterpret_cast<float2 *>(hold_all + (size_t)warps * 2 * n);
-    cs = CorrScratch{F_all + (size_t)warp * n * lds,
-                     reinterpret_cast<int *>(F_all + (size_t)warps * n * lds) + warp * 2 * n,
-                     hold};
-  }
+  float2 *F_all = reinterpret_cast<float2 *>(hold_all + (size_t)warps * 2 * n);
+  const CorrScratch cs{F_all + (size_t)warp * n * lds,
+                       reinterpret_cast<int *>(F_all + (size_t)warps * n * lds) + warp * 2 * n,
+                       hold};
   const int nn = n * n;
 
   // complex128 device batches: each matrix staged by bulk copies (bulk != 0),
@@ -84,12 +80,12 @@ __global__ void __launch_bounds__(kMaxWarpsPlain * 32)
       }
     }
     if (st < 0) st = src.load(b, n, M, lds, lane) ? LUFQHE_ST_NONFINITE : 0;
-    if (!st) st = lup_fp64_warp<ARITH>(M, lds, hold, n, lane, &par, CORRECT ? cs.ints : nullptr);
+    if (!st) st = lup_fp64_warp<ARITH_FUSED>(M, lds, hold, n, lane, &par, cs.ints);
 
     double la, ph;
     if (st == 0) {
       logdet_from_diag(M, lds, n, lane, par, &la, &ph);
-      if constexpr (CORRECT) fp64_correct_warp(src, b, n, M, lds, cs, lane, &la, &ph);
+      fp64_correct_warp(src, b, n, M, lds, cs, lane, &la, &ph);
     } else if (st == LUFQHE_ST_SINGULAR) {
       la = -INFINITY;
       ph = 0.0;
@@ -99,15 +95,82 @@ __global__ void __launch_bounds__(kMaxWarpsPlain * 32)
       par = 0;
     }
 
+    if (lane == 0) {
+      logabs[b] = la;
+      if (phase) phase[b] = ph;
+      if (parity) parity[b] = (int8_t)par;
+      if (status) status[b] = st | status_or;
+    }
+  }
+}
+
+// n <= 32, all but that route: 32 / LPM consecutive matrices per warp at a time
+// (lup_fp64_sub). Out: element type of the in-place factors (double2, or float2
+// for the reference's complex64 buffers).
+template <int ARITH, int LPM, class Src, class Out = double2>
+__global__ void __launch_bounds__(kMaxWarpsPlain * 32)
+    lup_plain_sub_kernel(Src src, Out *__restrict__ Aout, int n, int lda, long long batch,
+                         double *__restrict__ logabs, double *__restrict__ phase,
+                         int8_t *__restrict__ parity, int32_t *__restrict__ status,
+                         int status_or, int bulk) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int G = 32 / LPM;
+  const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int grp = lane / LPM, sub = lane % LPM;
+  const unsigned gmask = LPM == 32 ? kFull : ((1u << (LPM & 31)) - 1u) << (grp * LPM);
+  const int lds = n | 1;  // odd: a column read hits distinct banks
+  double2 *Mw = reinterpret_cast<double2 *>(smem_raw) + (size_t)warp * G * n * lds;
+  double2 *M = Mw + (size_t)grp * n * lds;
+  double *hold = reinterpret_cast<double *>(reinterpret_cast<double2 *>(smem_raw) +
+                                            (size_t)warps * G * n * lds) +
+                 (size_t)(warp * G + grp) * 2 * n;
+  constexpr bool BULK = std::is_same<Src, DenseSource>::value;
+  __shared__ __align__(8) uint64_t bars[kMaxWarpsPlain];
+  WarpBulk wb;
+  if constexpr (BULK)
+    if (bulk) wb.init(&bars[warp], lane);
+  const long long stride = (long long)gridDim.x * warps * G;
+  for (long long b0 = ((long long)blockIdx.x * warps + warp) * G; b0 < batch; b0 += stride) {
+    const int cnt = (int)min((long long)G, batch - b0);
+    const bool valid = grp < cnt;
+    __syncwarp();
+    int st = 0, par = 0;
+    bool staged = false;
+    if constexpr (BULK) {
+      if (bulk && !wb.broken) {
+        if (b0 + stride < batch && lane == 0)
+          prefetch_rows_l2(src.A + (size_t)(b0 + stride) * n * src.lda,
+                           (int)min((long long)G, batch - b0 - stride) * n, n, src.lda);
+        if (!wb.load_rows(src.A + (size_t)b0 * n * src.lda, cnt * n, n, src.lda, Mw, lds, n,
+                          lane))
+          st = LUFQHE_ST_WAIT_TIMEOUT;
+        staged = true;
+      }
+    }
+    if (!staged) load_rows(src, b0, cnt * n, n, Mw, lds, n, lane);
+    __syncwarp();
+    if (st == 0) st = lup_fp64_sub<ARITH, LPM>(M, lds, hold, n, sub, gmask, valid, &par);
+    double la, ph;
+    logdet_from_diag_sub<LPM>(M, lds, n, sub, valid && st == 0, par, &la, &ph);
+    if (st == LUFQHE_ST_SINGULAR) {
+      la = -INFINITY;
+      ph = 0.0;
+    } else if (st != 0) {
+      la = NAN;
+      ph = NAN;
+      par = 0;
+    }
+    if (!valid) continue;
+    const long long b = b0 + grp;
     if (Aout && (st == 0 || st == LUFQHE_ST_SINGULAR)) {
       Out *dst = Aout + (size_t)b * n * lda;
-      BlockWalk w(lane, n);
-      for (int e = lane; e < nn; e += 32) {
+      StrideWalk w(sub, LPM, n);
+      for (int e = sub; e < n * n; e += LPM) {
         store_entry(dst + (size_t)w.i * lda + w.k, M[w.i * lds + w.k]);
         w.next(n);
       }
     }
-    if (lane == 0) {
+    if (sub == 0) {
       logabs[b] = la;
       if (phase) phase[b] = ph;
       if (parity) parity[b] = (int8_t)par;
@@ -229,6 +292,33 @@ size_t plain_smem_per_warp(int n) {
   return (size_t)n * (n + 1) * sizeof(double2) + 2 * (size_t)n * sizeof(double);
 }
 
+template <int LPM, class Src, class Out>
+int launch_plain_sub(Src src, Out *Aout, int n, int lda, long long batch, int arith,
+                     double *logabs, double *phase, int8_t *parity, int32_t *status,
+                     cudaStream_t stream, int status_or) {
+  constexpr int G = 32 / LPM;
+  const int warps = sub_warps(n, LPM);
+  const size_t smem = sub_smem(n, LPM);
+  auto kern = arith == ARITH_REF ? lup_plain_sub_kernel<ARITH_REF, LPM, Src, Out>
+                                 : lup_plain_sub_kernel<ARITH_FUSED, LPM, Src, Out>;
+  int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)smem),
+                      "cudaFuncSetAttribute(plain sub)");
+  if (rc) return rc;
+  int per_sm = 0;
+  rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, smem),
+                  "occupancy(plain sub)");
+  if (rc) return rc;
+  const long long want = (batch + warps * G - 1) / (warps * G);
+  const long long cap = (long long)device_sm_count() * (per_sm < 1 ? 1 : per_sm);
+  const int grid = (int)(want < cap ? want : cap);
+  KernelTimer timer(arith == ARITH_REF ? "lup_plain_kernel_ref" : "lup_plain_kernel", n, stream);
+  kern<<<grid, warps * 32, smem, stream>>>(src, Aout, n, lda, batch, logabs, phase, parity, status,
+                                           status_or, bulk_for(src));
+  timer.stop();
+  return check_cuda(cudaGetLastError(), "lup_plain_sub_kernel launch");
+}
+
 template <class Src, class Out = double2>
 int launch_plain_src(Src src, Out *Aout, int n, int lda, long long batch, int arith,
                      double *logabs, double *phase, int8_t *parity, int32_t *status,
@@ -266,6 +356,22 @@ int launch_plain_src(Src src, Out *Aout, int n, int lda, long long batch, int ar
     timer.stop();
     return check_cuda(cudaGetLastError(), "lup_plain_group_kernel launch");
   }
+  if (!correct) {
+    switch (sub_lanes(n, batch, arith, device_sm_count(), device_smem_optin() + 1024)) {
+      case 4:
+        return launch_plain_sub<4>(src, Aout, n, lda, batch, arith, logabs, phase, parity, status,
+                                   stream, status_or);
+      case 8:
+        return launch_plain_sub<8>(src, Aout, n, lda, batch, arith, logabs, phase, parity, status,
+                                   stream, status_or);
+      case 16:
+        return launch_plain_sub<16>(src, Aout, n, lda, batch, arith, logabs, phase, parity,
+                                    status, stream, status_or);
+      default:
+        return launch_plain_sub<32>(src, Aout, n, lda, batch, arith, logabs, phase, parity,
+                                    status, stream, status_or);
+    }
+  }
   const size_t per_warp = plain_smem_per_warp(n) + (correct ? corr_smem : 0);
   const size_t optin = device_smem_optin();
   int warps = (int)(optin / per_warp);
@@ -276,9 +382,7 @@ int launch_plain_src(Src src, Out *Aout, int n, int lda, long long batch, int ar
     return LUFQHE_ERR_UNSUPPORTED_N;
   }
   const size_t smem = per_warp * warps;
-  auto kern = correct              ? lup_plain_kernel<ARITH_FUSED, Src, Out, true>
-              : arith == ARITH_REF ? lup_plain_kernel<ARITH_REF, Src, Out>
-                                   : lup_plain_kernel<ARITH_FUSED, Src, Out>;
+  auto kern = lup_plain_correct_kernel<Src>;
   int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)smem),
                       "cudaFuncSetAttribute(plain)");
@@ -291,11 +395,11 @@ int launch_plain_src(Src src, Out *Aout, int n, int lda, long long batch, int ar
   long long want = (batch + warps - 1) / warps;
   long long cap = (long long)device_sm_count() * per_sm;
   int grid = (int)(want < cap ? want : cap);
-  KernelTimer timer(arith == ARITH_REF ? "lup_plain_kernel_ref" : "lup_plain_kernel", n, stream);
-  kern<<<grid, warps * 32, smem, stream>>>(src, Aout, n, lda, batch, logabs, phase, parity, status,
-                                           status_or, bulk_for(src));
+  KernelTimer timer("lup_plain_kernel", n, stream);
+  kern<<<grid, warps * 32, smem, stream>>>(src, n, batch, logabs, phase, parity, status, status_or,
+                                           bulk_for(src));
   timer.stop();
-  return check_cuda(cudaGetLastError(), "lup_plain_kernel launch");
+  return check_cuda(cudaGetLastError(), "lup_plain_correct_kernel launch");
 }
 
 int launch_plain(const double2 *A, double2 *Aout, int n, int lda, long long batch, int arith,

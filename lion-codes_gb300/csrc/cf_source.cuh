@@ -24,7 +24,9 @@
 // The table and u, v are computed once per configuration on the host (cf.cu)
 // and read by every row. The sums are formed on the device, in a pre-pass of
 // one thread per row, with every operation explicitly rounded, so a host
-// restatement of the same operation order reproduces their bits. A
+// restatement of the same operation order reproduces their bits. A term depends
+// on its two particles only, so the batch's rows read the terms from an np x np
+// table (one pass over the pairs) where that is less work than forming each. A
 // permutation entry outside 1..np gives a NaN row (status NONFINITE), never a
 // read out of range; a repeated particle gives 0 * inf in its sums, also NaN.
 #pragma once
@@ -47,10 +49,28 @@ struct CfParams {
   int np;
   int cmu, cnu;        // table columns Q+1+mu, Q+1+nu
   double k1, k2, r1, r2;
+  // the pair terms of every two particles (np x np x 2, pair_terms), or nullptr
+  const double2 *pairs;
 
   __device__ __forceinline__ int particle(long long b, int r) const {
     const int p = (int)__ldg(perm + (size_t)b * pstride + r) - 1;
     return (p >= 0 && p < np) ? p : -1;
+  }
+  // The terms of particle q in the two sums of particle p.
+  __device__ __forceinline__ void pair_terms(double2 ui, double2 vi, int q, double2 &t1,
+                                             double2 &t2) const {
+    const double2 a = cd_mul(ui, __ldg(uv + np + q));
+    const double2 c = cd_mul(__ldg(uv + q), vi);
+    const double dx = __dsub_rn(a.x, c.x), dy = __dsub_rn(a.y, c.y);
+    const double w = __drcp_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
+    const double n1x = __dadd_rn(__dmul_rn(k1, a.x), __dmul_rn(k2, c.x));
+    const double n1y = __dadd_rn(__dmul_rn(k1, a.y), __dmul_rn(k2, c.y));
+    const double n2x = __dadd_rn(__dmul_rn(r1, a.x), __dmul_rn(r2, c.x));
+    const double n2y = __dadd_rn(__dmul_rn(r1, a.y), __dmul_rn(r2, c.y));
+    t1.x = __dmul_rn(__dadd_rn(__dmul_rn(n1x, dx), __dmul_rn(n1y, dy)), w);
+    t1.y = __dmul_rn(__dsub_rn(__dmul_rn(n1y, dx), __dmul_rn(n1x, dy)), w);
+    t2.x = __dmul_rn(__dadd_rn(__dmul_rn(n2x, dx), __dmul_rn(n2y, dy)), w);
+    t2.y = __dmul_rn(__dsub_rn(__dmul_rn(n2y, dx), __dmul_rn(n2x, dy)), w);
   }
   // Entries (r, n-2) and (r, n-1) of matrix b. Per pair (p, q):
   //   a = u_p v_q, c = u_q v_p, d = a - c, w = RN(1 / |d|^2),
@@ -62,23 +82,24 @@ struct CfParams {
     e1 = e2 = make_double2(NAN, NAN);
     if (p < 0) return;
     const double2 ui = __ldg(uv + p), vi = __ldg(uv + np + p);
+    const double2 *row = pairs ? pairs + (size_t)p * np * 2 : nullptr;
     double2 s1 = make_double2(0.0, 0.0), s2 = make_double2(0.0, 0.0);
+#pragma unroll 2
     for (int s = 0; s < n; ++s) {
       if (s == r) continue;
       const int q = particle(b, s);
       if (q < 0) return;
-      const double2 a = cd_mul(ui, __ldg(uv + np + q));
-      const double2 c = cd_mul(__ldg(uv + q), vi);
-      const double dx = __dsub_rn(a.x, c.x), dy = __dsub_rn(a.y, c.y);
-      const double w = __drcp_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
-      const double n1x = __dadd_rn(__dmul_rn(k1, a.x), __dmul_rn(k2, c.x));
-      const double n1y = __dadd_rn(__dmul_rn(k1, a.y), __dmul_rn(k2, c.y));
-      const double n2x = __dadd_rn(__dmul_rn(r1, a.x), __dmul_rn(r2, c.x));
-      const double n2y = __dadd_rn(__dmul_rn(r1, a.y), __dmul_rn(r2, c.y));
-      s1.x = __dadd_rn(s1.x, __dmul_rn(__dadd_rn(__dmul_rn(n1x, dx), __dmul_rn(n1y, dy)), w));
-      s1.y = __dadd_rn(s1.y, __dmul_rn(__dsub_rn(__dmul_rn(n1y, dx), __dmul_rn(n1x, dy)), w));
-      s2.x = __dadd_rn(s2.x, __dmul_rn(__dadd_rn(__dmul_rn(n2x, dx), __dmul_rn(n2y, dy)), w));
-      s2.y = __dadd_rn(s2.y, __dmul_rn(__dsub_rn(__dmul_rn(n2y, dx), __dmul_rn(n2x, dy)), w));
+      double2 t1, t2;
+      if (row) {
+        t1 = __ldg(row + 2 * q);
+        t2 = __ldg(row + 2 * q + 1);
+      } else {
+        pair_terms(ui, vi, q, t1, t2);
+      }
+      s1.x = __dadd_rn(s1.x, t1.x);
+      s1.y = __dadd_rn(s1.y, t1.y);
+      s2.x = __dadd_rn(s2.x, t2.x);
+      s2.y = __dadd_rn(s2.y, t2.y);
     }
     e1 = cd_mul(s1, __ldg(tab + (size_t)p * n + cmu));
     e2 = cd_mul(s2, __ldg(tab + (size_t)p * n + cnu));

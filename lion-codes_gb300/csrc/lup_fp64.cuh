@@ -445,24 +445,28 @@ struct NamedBarrier {
 };
 
 // The same factorisation by all threads of a warp group (a CTA, or part of
-// one behind a named barrier), for n > 32 where one warp per matrix leaves too
-// few warps on an SM to keep the FP64 pipe busy. Every pivot decision is taken
-// on the same candidate keys with the same rule (ties to the larger row) and
-// every entry sees the same operations in the same order as in lup_fp64_warp,
-// so the factors, pivots and parity are bit-identical to it. `red` is
-// 3 x (warps) words of shared scratch for the cross-warp reductions; tid and
-// nthr number the group's threads. Group-uniform return value.
+// one behind a named barrier), for n > 32 (at most 64) where one warp per matrix
+// leaves too few warps on an SM to keep the FP64 pipe busy. Every pivot decision
+// is taken on the same candidate keys with the same rule (ties to the larger
+// row) and every entry sees the same operations in the same order as in
+// lup_fp64_warp, so the factors, pivots and parity are bit-identical to it.
+// The pivot search and the multipliers of a column are one warp's (two rows per
+// lane) while the others exchange the rows: 3 barriers per column instead of 7,
+// and no search or division repeated on several warps. The columns take the
+// warps in turn, so that the SM sub-partitions share that work. us, before ->
+// now, fused / reference arithmetic: 2048 LLL x n=64 (6 warps) 1724 -> 1620 /
+// 3607 -> 3355, 4096 x n=48 1469 -> 1424 / 3326 -> 2968; the FP64 pipe is 80 to
+// 88% busy. `red` is at least 2 words of shared scratch; tid and nthr number the
+// group's threads (two warps or more). Group-uniform return value and parity.
 template <int ARITH, class Bar = CtaBarrier>
 __device__ int lup_fp64_group(double2 *M, int lds, double *hold, int n, int tid, int nthr,
                               long long *red, int *parity, Bar bar = Bar(), int *perm = nullptr) {
   const int lane = tid & 31, warp = tid >> 5, nw = nthr >> 5;
   if (perm)
     for (int i = tid; i < n; i += nthr) perm[i] = i;
-  long long *red_k = red;
-  int *red_i = reinterpret_cast<int *>(red + nw);
-  unsigned *red_n = reinterpret_cast<unsigned *>(red_i + nw);
   int par = 0;
   double *rhold = hold + n;
+  volatile int *pick = reinterpret_cast<volatile int *>(red);
   {
     bool tiny = false;
     const long long tiny_bits = __double_as_longlong(1e-24);
@@ -479,122 +483,150 @@ __device__ int lup_fp64_group(double2 *M, int lds, double *hold, int n, int tid,
       return LUFQHE_ST_SCALE_TINY;
     }
   }
-  // argmax over the CTA of (key, row), ties to the larger row
-  auto argmax = [&](long long &bk, int &bi) {
+  auto argmax = [](long long &bk, int &bi) {
 #pragma unroll
     for (int off = 16; off; off >>= 1) {
-      long long ok = __shfl_xor_sync(kFull, bk, off);
-      int oi = __shfl_xor_sync(kFull, bi, off);
+      const long long ok = __shfl_xor_sync(kFull, bk, off);
+      const int oi = __shfl_xor_sync(kFull, bi, off);
       if (ok > bk || (ok == bk && oi > bi)) {
         bk = ok;
         bi = oi;
       }
     }
-    if (lane == 0) {
-      red_k[warp] = bk;
-      red_i[warp] = bi;
-    }
-    bar.sync();
-    bk = red_k[0];
-    bi = red_i[0];
-    for (int q = 1; q < nw; ++q) {
-      if (red_k[q] > bk || (red_k[q] == bk && red_i[q] > bi)) {
-        bk = red_k[q];
-        bi = red_i[q];
-      }
-    }
-    bar.sync();
   };
+  const long long inf_bits = 0x7ff0000000000000ll;
   const long long safe_lo = 0x0170000000000000ll;  // 2^-1000
   const long long safe_hi = 0x7e70000000000000ll;  // 2^+1000
   for (int j = 0; j < n; ++j) {
-    long long bk = -1;
-    int bi = j;
-    for (int i = j + tid; i < n; i += nthr) {
-      double a = __dmul_rn(fabs(M[i * lds + j].x), rhold[i]);
-      long long key = (a == a) ? __double_as_longlong(a) : -2ll;
-      if (key >= bk) {
-        bk = key;
-        bi = i;
-      }
-    }
-    argmax(bk, bi);
-    unsigned near = 0;
-    for (int i = j + tid; i < n; i += nthr) {
-      double a = __dmul_rn(fabs(M[i * lds + j].x), rhold[i]);
-      long long key = (a == a) ? __double_as_longlong(a) : -2ll;
-      near += key >= bk - 16;
-    }
-    near = __reduce_add_sync(kFull, near);
-    if (lane == 0) red_n[warp] = near;
-    bar.sync();
-    near = 0;
-    for (int q = 0; q < nw; ++q) near += red_n[q];
-    bar.sync();
-    if (near != 1 || bk < safe_lo || bk > safe_hi) {
-      bk = -1;
-      bi = j;
-      for (int i = j + tid; i < n; i += nthr) {
-        double q = __ddiv_rn(fabs(M[i * lds + j].x), hold[i]);
-        long long key = (q == q) ? __double_as_longlong(q) : -2ll;
-        if (key >= bk) {
-          bk = key;
-          bi = i;
+    const int lead = j % nw;  // this column's warp
+    if (warp == lead) {
+      long long key[2], bk = -1;
+      int bi = j;
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int i = j + lane + 32 * q;
+        key[q] = -3;
+        if (j + 32 * q >= n) continue;  // no row of this slot
+        if (i < n) {
+          const long long a =
+              __double_as_longlong(__dmul_rn(fabs(M[i * lds + j].x), rhold[i]));
+          key[q] = (a & 0x7fffffffffffffffll) > inf_bits ? -2 : a;
+          if (key[q] >= bk) {
+            bk = key[q];
+            bi = i;
+          }
         }
       }
       argmax(bk, bi);
-    }
-    const int p = bi;
-    if (p != j) {
-      for (int k = tid; k < n; k += nthr) {
-        double2 t = M[p * lds + k];
-        M[p * lds + k] = M[j * lds + k];
-        M[j * lds + k] = t;
+      int near = 0;
+#pragma unroll
+      for (int q = 0; q < 2; ++q) near += __popc(__ballot_sync(kFull, key[q] >= bk - 16 && key[q] > -3));
+      if (near != 1 || bk < safe_lo || bk > safe_hi) {
+        bk = -1;
+        bi = j;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int i = j + lane + 32 * q;
+          if (i < n) {
+            const double d = __ddiv_rn(fabs(M[i * lds + j].x), hold[i]);
+            const long long k = (d == d) ? __double_as_longlong(d) : -2ll;
+            if (k >= bk) {
+              bk = k;
+              bi = i;
+            }
+          }
+        }
+        argmax(bk, bi);
       }
-      if (tid == 0) {
-        hold[p] = hold[j];
-        rhold[p] = rhold[j];
-        if (perm) {
-          const int t = perm[p];
-          perm[p] = perm[j];
-          perm[j] = t;
+      if (lane == 0) {
+        pick[0] = bi;
+        pick[1] = is_zero_c(M[bi * lds + j]);
+        if (bi != j) {
+          hold[bi] = hold[j];
+          rhold[bi] = rhold[j];
+          if (perm) {
+            const int t = perm[bi];
+            perm[bi] = perm[j];
+            perm[j] = t;
+          }
         }
       }
-      par ^= 1;
     }
     bar.sync();
-    const double2 piv = M[j * lds + j];
-    if (is_zero_c(piv)) {
+    const int p = pick[0];
+    const bool singular = pick[1] != 0;
+    par ^= p != j ? 1 : 0;
+    // rows p and j exchanged, column j (the leading warp's) aside
+    if (p != j && (warp != lead || singular))
+      for (int k = singular ? tid : (warp - (warp > lead ? 1 : 0)) * 32 + lane; k < n;
+           k += singular ? nthr : nthr - 32)
+        if (singular || k != j) {
+          const double2 t = M[p * lds + k];
+          M[p * lds + k] = M[j * lds + k];
+          M[j * lds + k] = t;
+        }
+    if (singular) {
+      bar.sync();
       *parity = par;
       return LUFQHE_ST_SINGULAR;
     }
     if (j == n - 1) break;
-    if (ARITH == ARITH_REF) {
-      const double den = pivot_den<ARITH_REF>(piv);
-      const double y = __drcp_rn(den);
-      const long long db = abs_bits(den);
-      const bool den_safe = db >= 0x03f0000000000000ll && db <= 0x7bf0000000000000ll;
-      for (int i = j + 1 + tid; i < n; i += nthr) {
-        const double2 a = M[i * lds + j];
-        const double nx = __dadd_rn(__dmul_rn(a.x, piv.x), __dmul_rn(a.y, piv.y));
-        const double ny = __dsub_rn(__dmul_rn(a.y, piv.x), __dmul_rn(a.x, piv.y));
-        M[i * lds + j] = make_double2(div_rn_markstein(nx, den, y, den_safe),
-                                      div_rn_markstein(ny, den, y, den_safe));
+    if (warp == lead) {
+      const double2 piv = M[p * lds + j], top = M[j * lds + j];
+      double2 a[2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int i = j + 1 + lane + 32 * q;
+        a[q] = i == p ? top : i < n ? M[i * lds + j] : make_double2(0.0, 0.0);
       }
-    } else {
-      const double d = pivot_den<ARITH>(piv);
-      for (int i = j + 1 + tid; i < n; i += nthr)
-        M[i * lds + j] = cdiv_pivot<ARITH>(M[i * lds + j], piv, d);
+      __syncwarp();
+      if (lane == 0) M[j * lds + j] = piv;
+      const double den = pivot_den<ARITH>(piv);
+      double y = 0.0;
+      bool den_safe = false;
+      if (ARITH == ARITH_REF) {
+        y = __drcp_rn(den);
+        const long long db = abs_bits(den);
+        den_safe = db >= 0x03f0000000000000ll && db <= 0x7bf0000000000000ll;  // [2^-960, 2^960]
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int i = j + 1 + lane + 32 * q;
+        if (j + 1 + 32 * q >= n) continue;
+        if (i < n) {
+          if (ARITH == ARITH_REF) {
+            const double nx = __dadd_rn(__dmul_rn(a[q].x, piv.x), __dmul_rn(a[q].y, piv.y));
+            const double ny = __dsub_rn(__dmul_rn(a[q].y, piv.x), __dmul_rn(a[q].x, piv.y));
+            M[i * lds + j] = make_double2(div_rn_markstein(nx, den, y, den_safe),
+                                          div_rn_markstein(ny, den, y, den_safe));
+          } else {
+            M[i * lds + j] = cdiv_pivot<ARITH>(a[q], piv, den);
+          }
+        }
+      }
     }
     bar.sync();
     const int m = n - 1 - j;
     const int mm = m * m;
-    const int j1 = j + 1;
+    double2 *T = M + (j + 1) * lds + j + 1;
+    const double2 *L = M + (j + 1) * lds + j, *U = M + j * lds + j + 1;
     StrideWalk w(tid, nthr, m);
-    for (int e = tid; e < mm; e += nthr) {
-      const int ii = j1 + w.i, kk = j1 + w.k;
-      M[ii * lds + kk] = cmsub<ARITH>(M[ii * lds + kk], M[ii * lds + j], M[j * lds + kk]);
+    for (int e = tid; e < mm; e += 2 * nthr) {
+      const int i0 = w.i, k0 = w.k;
       w.next(m);
+      const int i1 = w.i, k1 = w.k;
+      w.next(m);
+      if (e - lane + nthr < mm) {  // warp-uniform: two entries, one's loads over the other's work
+        const bool on = e + nthr < mm;
+        const int f1 = on ? i1 * lds + k1 : 0;
+        const double2 s0 = T[i0 * lds + k0], l0 = L[i0 * lds], u0 = U[k0];
+        const double2 s1 = T[f1], l1 = L[on ? i1 * lds : 0], u1 = U[on ? k1 : 0];
+        const double2 r0 = cmsub<ARITH>(s0, l0, u0), r1 = cmsub<ARITH>(s1, l1, u1);
+        T[i0 * lds + k0] = r0;
+        if (on) T[f1] = r1;
+      } else {
+        T[i0 * lds + k0] = cmsub<ARITH>(T[i0 * lds + k0], L[i0 * lds], U[k0]);
+      }
     }
     bar.sync();
   }

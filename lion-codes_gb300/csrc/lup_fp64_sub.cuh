@@ -27,7 +27,7 @@ namespace lufqhe {
 template <int ARITH, int LPM>
 __device__ int lup_fp64_sub(double2 *M, int lds, double *hold, int n, int sub, unsigned gmask,
                             bool valid, int *parity) {
-  constexpr int R = LPM == 32 ? 1 : 2;  // rows per lane
+  constexpr int R = 2;  // rows per lane (n <= 32 has one with 32 lanes)
   double *rhold = hold + n;
   int par = 0, st = 0;
   {
@@ -72,9 +72,10 @@ __device__ int lup_fp64_sub(double2 *M, int lds, double *hold, int n, int sub, u
     int bi = j;
 #pragma unroll
     for (int q = 0; q < R; ++q) {
-      const int i = sub + LPM * q;
+      const int i = j + sub + LPM * q;
       key[q] = -3;
-      if (live && i >= j && i < n) {
+      if (j + LPM * q >= n) continue;  // no row of this slot
+      if (live && i < n) {
         const long long a =
             __double_as_longlong(__dmul_rn(fabs(M[i * lds + j].x), rhold[i]));
         key[q] = (a & 0x7fffffffffffffffll) > inf_bits ? -2 : a;
@@ -87,18 +88,16 @@ __device__ int lup_fp64_sub(double2 *M, int lds, double *hold, int n, int sub, u
     argmax(bk, bi);
     int near = 0;
 #pragma unroll
-    for (int q = 0; q < R; ++q) {
-      const int i = sub + LPM * q;
-      near += __popc(__ballot_sync(kFull, live && i >= j && i < n && key[q] >= bk - 16) & gmask);
-    }
+    for (int q = 0; q < R; ++q)
+      near += __popc(__ballot_sync(kFull, key[q] > -3 && key[q] >= bk - 16) & gmask);
     const bool exact = live && (near != 1 || bk < safe_lo || bk > safe_hi);
     if (__any_sync(kFull, exact)) {
       long long ek = -1;
       int ei = j;
 #pragma unroll
       for (int q = 0; q < R; ++q) {
-        const int i = sub + LPM * q;
-        if (exact && i >= j && i < n) {
+        const int i = j + sub + LPM * q;
+        if (exact && i < n) {
           const double d = __ddiv_rn(fabs(M[i * lds + j].x), hold[i]);
           const long long k = (d == d) ? __double_as_longlong(d) : -2ll;
           if (k >= ek) {
@@ -188,7 +187,7 @@ __device__ __forceinline__ void logdet_from_diag_sub(const double2 *M, int lds, 
                                                      double *ph_out) {
   double la[2] = {0.0, 0.0}, ph[2] = {0.0, 0.0};
 #pragma unroll
-  for (int q = 0; q < (LPM == 32 ? 1 : 2); ++q) {
+  for (int q = 0; q < 2; ++q) {
     const int j = sub + LPM * q;
     if (live && j < n) {
       double lg, ar;

@@ -207,23 +207,29 @@ __global__ void write_det_kernel(T *A, int n, int lda, long long batch,
 
 }  // namespace
 
-// n > 32: one matrix per CTA of kGroupWarps warps (lup_fp64_group). With one
+// n > 32: one matrix per CTA of group_warps(n) warps (lup_fp64_group). With one
 // warp per matrix an SM holds only the 3-4 matrices its shared memory fits
 // (n=64: 66 KB each), too few warps to cover the FP64 pipe's latency.
-constexpr int kGroupWarps = kFp64GroupWarps;
+constexpr int kGroupMaxWarps = 6;
 constexpr int kGroupMinN = kFp64GroupMinN;
+// 4 warps up to n = 48, 6 above, where an SM holds 3 or 4 matrices only (2048
+// LLL x n=64, fused, us with 4 / 5 / 6 / 8 warps: 1745 / 1620 / 1621 / 1615;
+// reference arithmetic 3592 / 3395 / 3354 / 3410; 4096 x n=48 fused 1424 / 1425 /
+// 1431 / 1471).
+constexpr int kWarpMaxN = 40;
+constexpr int group_warps(int n) { return n > 48 ? kGroupMaxWarps : kFp64GroupWarps; }
 
 // CORRECT: the mixed mode's FP64 route, whose log-determinants get the
 // extended-precision correction (fp64_correct_group; its scratch follows the
 // row scales in shared memory).
 template <int ARITH, class Src, class Out = double2, bool CORRECT = false>
-__global__ void __launch_bounds__(kGroupWarps * 32)
+__global__ void __launch_bounds__(kGroupMaxWarps * 32)
     lup_plain_group_kernel(Src src, Out *__restrict__ Aout, int n, int lda, long long batch,
                            double *__restrict__ logabs, double *__restrict__ phase,
                            int8_t *__restrict__ parity, int32_t *__restrict__ status,
                            int status_or) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ long long red[3 * kGroupWarps];
+  __shared__ long long red[3 * kGroupMaxWarps];
   const int tid = threadIdx.x, nthr = blockDim.x;
   const int lds = n + 1;
   double2 *M = reinterpret_cast<double2 *>(smem_raw);
@@ -328,7 +334,19 @@ int launch_plain_src(Src src, Out *Aout, int n, int lda, long long batch, int ar
   const bool correct = status_or != 0 && arith == ARITH_FUSED && Aout == nullptr &&
                        n >= kCorrectMinN && n <= kCorrectMaxN;
   const size_t corr_smem = (size_t)n * (n + 1) * sizeof(float2) + 2 * (size_t)n * sizeof(int);
-  if (n >= kGroupMinN) {
+  // fused, n <= kWarpMaxN, a batch that fills its rounds of a warp per matrix:
+  // no barriers (8192 LLL x n=33 1055 us against 1163 by groups, x n=36 1310
+  // against 1405, 4096 x n=40 899 against 903; reference arithmetic 2219 against
+  // 2211; a part-filled round costs a whole one: 1900 x n=33 344 against 300)
+  bool warp_each = false;
+  if (n >= kGroupMinN && n <= kWarpMaxN && !correct && arith == ARITH_FUSED) {
+    const long long round = 4ll * (long long)((device_smem_optin() + 1024) /
+                                              (sub_smem(n, 32) + 1024)) * device_sm_count();
+    const long long rounds = (batch + round - 1) / round;
+    warp_each = 100 * batch >= 85 * rounds * round;
+  }
+  if (n >= kGroupMinN && !warp_each) {
+    const int threads = group_warps(n) * 32;
     const size_t smem = (size_t)n * (n + 1) * sizeof(double2) + 2 * (size_t)n * sizeof(double) +
                         (correct ? corr_smem : 0);
     auto kern = correct              ? lup_plain_group_kernel<ARITH_FUSED, Src, Out, true>
@@ -339,8 +357,7 @@ int launch_plain_src(Src src, Out *Aout, int n, int lda, long long batch, int ar
                         "cudaFuncSetAttribute(plain group)");
     if (rc) return rc;
     int per_sm = 0;
-    rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kGroupWarps * 32,
-                                                                  smem),
+    rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem),
                     "occupancy(plain group)");
     if (rc) return rc;
     if (per_sm < 1) {
@@ -351,7 +368,7 @@ int launch_plain_src(Src src, Out *Aout, int n, int lda, long long batch, int ar
     const int grid = (int)(batch < cap ? batch : cap);
     KernelTimer timer(arith == ARITH_REF ? "lup_plain_group_kernel_ref" : "lup_plain_group_kernel",
                       n, stream);
-    kern<<<grid, kGroupWarps * 32, smem, stream>>>(src, Aout, n, lda, batch, logabs, phase, parity,
+    kern<<<grid, threads, smem, stream>>>(src, Aout, n, lda, batch, logabs, phase, parity,
                                                    status, status_or);
     timer.stop();
     return check_cuda(cudaGetLastError(), "lup_plain_group_kernel launch");

@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "mixed_core.cuh"
+#include "mixed_grid.cuh"
 
 namespace lufqhe {
 
@@ -75,9 +76,7 @@ struct PlanAux {
 constexpr int kPlanDeferMinN = 24;
 
 // A plan's passes (see Launch), and the largest n of a mixed plan's small
-// pass: its own build of the grouped kernel, whose register-tiled cases stop
-// at n = 16, takes under 128 registers and runs two 8-warp CTAs per SM where
-// the build with the n = 24 and 32 cases (190 registers) runs one.
+// pass (grouped_small_kernel: the lane-grid path, several matrices per warp).
 constexpr int kPlanPasses = 4;
 constexpr int kSmallPassMaxN = 16;
 
@@ -137,7 +136,7 @@ __device__ void plan_fp64(const double2 *src, int n, int lda, long long ob, doub
                     status, flag, &cs, fl);
 }
 
-template <int MODE, bool SMALL = false>
+template <int MODE>
 __device__ void process_matrix(const double2 *src, int n, int lda, long long ob, float4 *HL,
                                float2 *F, double *hold, int *er, int *ec, int nm, int lane,
                                float theta2, bool refine, unsigned int share64k, int status_or,
@@ -164,19 +163,9 @@ __device__ void process_matrix(const double2 *src, int n, int lda, long long ob,
     float2 corr;
     bool ok;
     switch (n) {
-      case 6: ok = mixed_factor_tile<6>(HL, F, er, ec, lane, theta2, prod, exp_sum, corr, par, refine); break;
-      case 8: ok = mixed_factor_tile<8>(HL, F, er, ec, lane, theta2, prod, exp_sum, corr, par, refine); break;
-      case 12: ok = mixed_factor_tile<12>(HL, F, er, ec, lane, theta2, prod, exp_sum, corr, par, refine); break;
-      case 16: ok = mixed_factor_tile<16>(HL, F, er, ec, lane, theta2, prod, exp_sum, corr, par, refine); break;
-      // (never reached in the small pass, n <= kSmallPassMaxN)
-      case 24:
-        if constexpr (SMALL) ok = false;
-        else ok = mixed_factor_tile<24>(HL, F, er, ec, lane, theta2, prod, exp_sum, corr, par, refine);
-        break;
-      case 32:
-        if constexpr (SMALL) ok = false;
-        else ok = mixed_factor_tile<32>(HL, F, er, ec, lane, theta2, prod, exp_sum, corr, par, refine);
-        break;
+      // (n <= kSmallPassMaxN goes to the small pass)
+      case 24: ok = mixed_factor_tile<24>(HL, F, er, ec, lane, theta2, prod, exp_sum, corr, par, refine); break;
+      case 32: ok = mixed_factor_tile<32>(HL, F, er, ec, lane, theta2, prod, exp_sum, corr, par, refine); break;
       default: {
         MixedSmem S;
         S.SC = HL;
@@ -223,8 +212,8 @@ __device__ void process_matrix(const double2 *src, int n, int lda, long long ob,
   }
 }
 
-template <int MODE, bool SMALL = false>
-__global__ void __launch_bounds__(kMaxWarpsMixed * 32, SMALL ? 2 : 1)
+template <int MODE>
+__global__ void __launch_bounds__(kMaxWarpsMixed * 32)
     grouped_kernel(const WorkItem *__restrict__ items, int nitems, unsigned int *counter, int nm,
                    int nf,
                    float theta2, int refine, double *__restrict__ logabs, double *__restrict__ phase,
@@ -256,9 +245,74 @@ __global__ void __launch_bounds__(kMaxWarpsMixed * 32, SMALL ? 2 : 1)
     for (int j = 0; j < w.count; ++j) {
       __syncwarp();
       const long long b = w.first + j;
-      process_matrix<MODE, SMALL>(w.A + (size_t)b * w.n * w.lda, w.n, w.lda, w.out + j, HL, F, hold, er,
+      process_matrix<MODE>(w.A + (size_t)b * w.n * w.lda, w.n, w.lda, w.out + j, HL, F, hold, er,
                            ec, nm, lane, theta2, refine != 0, w.share64k, w.status_or, fl, aux,
                            out, logabs, phase, parity, status);
+    }
+  }
+  out.flush(lane, logabs, phase, parity, status);
+}
+
+// A mixed plan's small pass: the FP32-path groups with n <= kSmallPassMaxN, each
+// warp taking an item's matrices several at a time (the batched call's path and
+// bits). nm sizes a warp's shared memory.
+__host__ __device__ constexpr size_t small_warp_bytes(int nm) {
+  return nm <= 8 ? Grid<8, 8>::kWarpBytes
+         : nm <= 12 ? (Grid<12, 16>::kWarpBytes > Grid<8, 8>::kWarpBytes
+                           ? Grid<12, 16>::kWarpBytes
+                           : Grid<8, 8>::kWarpBytes)
+                    : Grid<16, 16>::kWarpBytes;
+}
+
+template <int NP, int LPM, int NC>
+__device__ void small_item(const WorkItem &w, unsigned char *base, int lane, float theta2,
+                           bool refine, DeferredOut &out, double *logabs, double *phase,
+                           int8_t *parity, int32_t *status) {
+  using Gd = Grid<NP, LPM>;
+  float4 *HLw = reinterpret_cast<float4 *>(base);
+  float2 *Fw = reinterpret_cast<float2 *>(HLw + Gd::G * Gd::kHL);
+  int *Iw = reinterpret_cast<int *>(Fw + Gd::G * Gd::kF);
+  const DenseSource src{w.A, w.lda};
+  const int n = NC ? NC : w.n;
+  for (int j = 0; j < w.count; j += Gd::G) {
+    const int cnt = min(Gd::G, w.count - j);
+    __syncwarp();
+    load_rows(src, w.first + j, cnt * n, n, reinterpret_cast<double2 *>(HLw), Gd::LDH, NP, lane);
+    __syncwarp();
+    grid_unit<NP, LPM, NC, true, true>(src, w.first + j, w.out + j, cnt, n, HLw, Fw, Iw, lane, theta2,
+                                 w.share64k, refine, [](long long, bool) {}, out, logabs, phase,
+                                 parity, status);
+  }
+}
+
+__global__ void __launch_bounds__(kMaxWarpsMixed * 32, 2)
+    grouped_small_kernel(const WorkItem *__restrict__ items, int nitems, unsigned int *counter,
+                         int nm, int nf, float theta2, int refine, double *__restrict__ logabs,
+                         double *__restrict__ phase, int8_t *__restrict__ parity,
+                         int32_t *__restrict__ status, PlanAux aux) {
+  (void)nf;
+  (void)aux;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  unsigned char *base = smem_raw + (size_t)warp * small_warp_bytes(nm);
+  DeferredOut out;
+  for (;;) {
+    unsigned int it = 0;
+    if (lane == 0) it = atomicAdd(counter, 1u);
+    it = __shfl_sync(kFull, it, 0);
+    if (it >= (unsigned int)nitems) break;
+    const WorkItem w = items[it];
+    const bool rf = refine != 0;
+    switch (w.n) {
+      case 6: small_item<8, 8, 6>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
+      case 8: small_item<8, 8, 8>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
+      case 12: small_item<12, 16, 12>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
+      case 16: small_item<16, 16, 16>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
+      default:
+        if (w.n < 8)
+          small_item<8, 8, 0>(w, base, lane, theta2, rf, out, logabs, phase, parity, status);
+        else
+          small_item<16, 16, 0>(w, base, lane, theta2, rf, out, logabs, phase, parity, status);
     }
   }
   out.flush(lane, logabs, phase, parity, status);
@@ -272,12 +326,16 @@ GroupedKernel kernel_for(int mode, bool small = false) {
     case LUFQHE_MODE_PLAIN_FP64: return grouped_kernel<LUFQHE_MODE_PLAIN_FP64>;
     case LUFQHE_MODE_PLAIN_FP64_FUSED: return grouped_kernel<LUFQHE_MODE_PLAIN_FP64_FUSED>;
     default:
-      return small ? grouped_kernel<LUFQHE_MODE_MIXED, true> : grouped_kernel<LUFQHE_MODE_MIXED>;
+      return small ? grouped_small_kernel : grouped_kernel<LUFQHE_MODE_MIXED>;
   }
 }
 
-// Default tile: about 64 n=8-equivalents of work per item (flops scale ~n^3).
-int default_tile(int n) {
+// Default tile: about 64 n=8-equivalents of work per item (flops scale ~n^3);
+// in a mixed plan's small pass two of a warp's units (a claim costs a tenth of a
+// unit, and a group of 7000 matrices of n = 6 in items of 152 had kept 46 of
+// 2432 warps busy).
+int default_tile(int n, int mode) {
+  if (mode == LUFQHE_MODE_MIXED && n <= kSmallPassMaxN) return n <= 8 ? 8 : 4;
   double t = 64.0 * std::pow(8.0 / (double)n, 3.0);
   int v = (int)std::lround(t);
   return std::max(1, std::min(256, v));
@@ -411,8 +469,8 @@ GroupedKernel group_kernel_for(int mode, bool correct) {
 //     the precision policy sends to FP64;
 //  2. the warp-group kernel over the FP64-route groups with n > 32 (fused
 //     arithmetic for a mixed plan, the plan's arithmetic for a plain one);
-//  3. (mixed plans) the small build of the mixed kernel over the FP32-path
-//     groups with n <= kSmallPassMaxN, at twice pass 0's occupancy.
+//  3. (mixed plans) grouped_small_kernel over the FP32-path groups with
+//     n <= kSmallPassMaxN.
 // Groups routed to FP64 need neither the FP32 path's shared memory nor its
 // registers, and get the plain kernels' occupancy. After the passes a mixed
 // plan runs its pending pass (grouped_pending_kernel) and the correction
@@ -588,7 +646,7 @@ int configure_pass(lufqhe_plan_s *p, int pass, int warps) {
     return LUFQHE_SUCCESS;
   }
   GroupedKernel k = kernel_for(L.mode, pass == 3);
-  const size_t per_warp = warp_layout(L.nm, L.nf).total;
+  const size_t per_warp = pass == 3 ? small_warp_bytes(L.nm) : warp_layout(L.nm, L.nf).total;
   const size_t optin = device_smem_optin();
   int w = std::min<int>(warps, (int)(optin / per_warp));
   if (w < 1) {
@@ -916,7 +974,7 @@ extern "C" int lufqhe_plan_create(lufqhe_plan_t **plan, const lufqhe_group_t *gr
     }
     p->groups.push_back(G);
     p->groups.back().A = device_address(G.A);
-    p->tile.push_back(default_tile(G.n));
+    p->tile.push_back(default_tile(G.n, p->mode));
     // the per-n FP64 share of the batched mixed kernels
     p->share.push_back(fp64_share_64k(G.n));
     p->nmax = std::max(p->nmax, G.n);

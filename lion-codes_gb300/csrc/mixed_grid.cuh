@@ -615,6 +615,118 @@ __device__ __forceinline__ int grid_factor(float4 *HL, float2 *F, int *ints, con
   return code;
 }
 
+// F of one matrix from the grid path's row stride to stride N + 1, in place.
+template <int NP, int N>
+__device__ __forceinline__ void repack_f(float2 *F, int lane) {
+  constexpr int K = (N * N + 31) / 32;
+  float2 v[K];
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < K; ++q) {
+    const int e = lane + 32 * q;
+    if (e < N * N) v[q] = F[e / N * (NP + 2) + e % N];
+  }
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < K; ++q) {
+    const int e = lane + 32 * q;
+    if (e < N * N) F[e / N * (N + 1) + e % N] = v[q];
+  }
+  __syncwarp();
+}
+
+// FP64 refactorisation of matrix sb of src into output ob, in one matrix's area
+// of the lane grid, by the whole warp. Sizes up to 16 have no correction, so the
+// row scales may lie over F where no padding is left after the matrix (n = NP).
+template <int NP, class Src>
+__device__ __forceinline__ void grid_refactor(const Src &src, long long sb, int n, float4 *HL,
+                                              float2 *F, int lane, long long ob, double *logabs,
+                                              double *phase, int8_t *parity, int32_t *status,
+                                              int flag) {
+  double *hold = n < NP ? reinterpret_cast<double *>(HL + (size_t)n * (n + 1))
+                        : reinterpret_cast<double *>(F);
+  fallback_fp64_src(src, sb, n, reinterpret_cast<double2 *>(HL), n + 1, hold, lane, ob, logabs,
+                    phase, parity, status, flag);
+}
+// The same out of line, for a kernel with many sizes. (In the batched kernels
+// the call cost more than the code it saves: 65536 LLL x n=16 645 -> 677 us.)
+template <int NP, class Src>
+__device__ __noinline__ void grid_refactor_call(const Src src, long long sb, int n, float4 *HL,
+                                                float2 *F, int lane, long long ob, double *logabs,
+                                                double *phase, int8_t *parity, int32_t *status,
+                                                int flag) {
+  grid_refactor<NP>(src, sb, n, HL, F, lane, ob, logabs, phase, parity, status, flag);
+}
+
+// The `cnt` matrices from b0 of src, staged in the warp's area (group q at
+// HLw + q kHL), into outputs ob0 ..: the FP32 path, then what it does not accept:
+// refined or refactorised right here (INPLACE, n <= 16), or handed to
+// defer(b, routed). share64k: the share routed straight to FP64. CALL: FP64 out
+// of line.
+template <int NP, int LPM, int NC, bool INPLACE, bool CALL, class Src, class Defer>
+__device__ __forceinline__ void grid_unit(const Src &src, long long b0, long long ob0, int cnt,
+                                          int n, float4 *HLw, float2 *Fw, int *Iw, int lane,
+                                          float theta2, unsigned int share64k, bool refine,
+                                          Defer defer, DeferredOut &out, double *logabs,
+                                          double *phase, int8_t *parity, int32_t *status) {
+  using Gd = Grid<NP, LPM>;
+  const int grp = lane / LPM;
+  CFF prod;
+  int exp_sum, par;
+  float2 corr;
+  int code = grid_factor<NP, LPM, NC, INPLACE>(HLw + grp * Gd::kHL, Fw + grp * Gd::kF,
+                                               Iw + grp * 2 * NP, n, lane, theta2, prod, exp_sum,
+                                               corr, par);
+  bool routed = false;
+  if (share64k && grp < cnt && code != TILE_NONFINITE) {
+    routed = route_fp64_entry(src.first(b0 + grp, n), share64k);
+    if (routed) code = TILE_REJECT;
+  }
+#pragma unroll 1
+  for (int q = 0; q < cnt; ++q) {
+    const int from = q * LPM;
+    const int cq = __shfl_sync(kFull, code, from);
+    const CFF pq = shfl_cff(prod, from, false);
+    const int eq = __shfl_sync(kFull, exp_sum, from);
+    const int rq = __shfl_sync(kFull, par, from);
+    float2 kq = shfl2(corr, from);
+    const long long ob = ob0 + q;
+    if (cq == TILE_ACCEPT) {
+      out.push(lane, ob, pq, eq, kq, rq, logabs, phase, parity, status);
+      continue;
+    }
+    if (cq == TILE_NONFINITE) {
+      emit_nonfinite(lane, ob, logabs, phase, parity, status);
+      continue;
+    }
+    const bool rt = __shfl_sync(kFull, (int)routed, from) != 0;
+    if constexpr (!INPLACE) {
+      defer(b0 + q, rt);
+    } else {
+      float4 *HLq = HLw + q * Gd::kHL;
+      float2 *Fq = Fw + q * Gd::kF;
+      if constexpr (NC != 0) {
+        if (cq == TILE_REFINE && refine) {
+          float2 *Rm = reinterpret_cast<float2 *>(HLq);
+          repack_f<NP, NC>(Fq, lane);
+          if (mixed_refine_tile<NC>(Fq, Rm, Rm + NC * (NC + 1),
+                                    reinterpret_cast<float2 *>(Iw + q * 2 * NP), lane, theta2,
+                                    tile_la_est(pq, eq), kq)) {
+            out.push(lane, ob, pq, eq, kq, rq, logabs, phase, parity, status);
+            continue;
+          }
+        }
+      }
+      const int flag = rt ? LUFQHE_ST_FP64 : LUFQHE_ST_FALLBACK;
+      if constexpr (CALL)
+        grid_refactor_call<NP>(src, b0 + q, n, HLq, Fq, lane, ob, logabs, phase, parity, status,
+                               flag);
+      else
+        grid_refactor<NP>(src, b0 + q, n, HLq, Fq, lane, ob, logabs, phase, parity, status, flag);
+    }
+  }
+}
+
 }  // namespace
 }  // namespace mixed
 }  // namespace lufqhe

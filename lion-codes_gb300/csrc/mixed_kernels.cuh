@@ -252,26 +252,6 @@ __global__ void __launch_bounds__(kMaxWarpsMixed * 32)
 }
 
 
-// F of one matrix from the grid path's row stride to stride N + 1, in place.
-template <int NP, int N>
-__device__ __forceinline__ void repack_f(float2 *F, int lane) {
-  constexpr int K = (N * N + 31) / 32;
-  float2 v[K];
-  __syncwarp();
-#pragma unroll
-  for (int q = 0; q < K; ++q) {
-    const int e = lane + 32 * q;
-    if (e < N * N) v[q] = F[e / N * (NP + 2) + e % N];
-  }
-  __syncwarp();
-#pragma unroll
-  for (int q = 0; q < K; ++q) {
-    const int e = lane + 32 * q;
-    if (e < N * N) F[e / N * (N + 1) + e % N] = v[q];
-  }
-  __syncwarp();
-}
-
 // The FP32 pass of the lane-grid path: each warp takes Grid::G consecutive
 // matrices at a time. NC = n for the register-tiled sizes, 0 for the generic
 // rule. DEFER: rejected matrices go to the call's pending list; else they are
@@ -287,7 +267,6 @@ __global__ void __launch_bounds__(grid_warps(NP) * 32, grid_min_ctas(NP))
   constexpr bool BULK = std::is_same<Src, DenseSource>::value;
   const int n = NC ? NC : n_rt;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int grp = lane / LPM;
   unsigned char *base = smem_raw + (size_t)warp * Gd::kWarpBytes;
   float4 *HLw = reinterpret_cast<float4 *>(base);
   float2 *Fw = reinterpret_cast<float2 *>(HLw + Gd::G * Gd::kHL);
@@ -324,62 +303,10 @@ __global__ void __launch_bounds__(grid_warps(NP) * 32, grid_min_ctas(NP))
     }
     if (!staged) load_rows(src, b0, cnt * n, n, M, Gd::LDH, NP, lane);
     __syncwarp();
-    CFF prod;
-    int exp_sum, par;
-    float2 corr;
-    int code = grid_factor<NP, LPM, NC, !DEFER>(HLw + grp * Gd::kHL, Fw + grp * Gd::kF,
-                                                Iw + grp * 2 * NP, n, lane, theta2, prod, exp_sum,
-                                                corr, par);
-    bool routed = false;
-    if (share64k && grp < cnt && code != TILE_NONFINITE) {
-      routed = route_fp64_entry(src.first(b0 + grp, n), share64k);
-      if (routed) code = TILE_REJECT;
-    }
-#pragma unroll 1
-    for (int q = 0; q < cnt; ++q) {
-      const int from = q * LPM;
-      const int cq = __shfl_sync(kFull, code, from);
-      const CFF pq = shfl_cff(prod, from, false);
-      const int eq = __shfl_sync(kFull, exp_sum, from);
-      const int rq = __shfl_sync(kFull, par, from);
-      float2 kq = shfl2(corr, from);
-      const long long b = b0 + q;
-      if (cq == TILE_ACCEPT) {
-        out.push(lane, b, pq, eq, kq, rq, logabs, phase, parity, status);
-        continue;
-      }
-      if (cq == TILE_NONFINITE) {
-        emit_nonfinite(lane, b, logabs, phase, parity, status);
-        continue;
-      }
-      const bool rt = __shfl_sync(kFull, (int)routed, from) != 0;
-      if constexpr (DEFER) {
-        defer_fp64(head, pend, b, lane, rt);
-      } else {
-        float4 *HLq = HLw + q * Gd::kHL;
-        float2 *Fq = Fw + q * Gd::kF;
-        int *Iq = Iw + q * 2 * NP;
-        if constexpr (NC != 0) {
-          if (cq == TILE_REFINE && refine) {
-            float2 *Rm = reinterpret_cast<float2 *>(HLq);
-            repack_f<NP, NC>(Fq, lane);
-            if (mixed_refine_tile<NC>(Fq, Rm, Rm + NC * (NC + 1), reinterpret_cast<float2 *>(Iq),
-                                      lane, theta2, tile_la_est(pq, eq), kq)) {
-              out.push(lane, b, pq, eq, kq, rq, logabs, phase, parity, status);
-              continue;
-            }
-          }
-        }
-        // the matrix again in this group's area, its row scales after it where
-        // the padding leaves room (n < NP), else over F (sizes up to 16 have no
-        // correction, which would use F)
-        double *hold = n < NP ? reinterpret_cast<double *>(HLq + (size_t)n * (n + 1))
-                              : reinterpret_cast<double *>(Fq);
-        fallback_fp64_src(src, b, n, reinterpret_cast<double2 *>(HLq), n + 1, hold, lane, b,
-                          logabs, phase, parity, status,
-                          rt ? LUFQHE_ST_FP64 : LUFQHE_ST_FALLBACK);
-      }
-    }
+    grid_unit<NP, LPM, NC, !DEFER, false>(
+        src, b0, b0, cnt, n, HLw, Fw, Iw, lane, theta2, share64k, refine != 0,
+        [&](long long b, bool routed) { defer_fp64(head, pend, b, lane, routed); }, out, logabs,
+        phase, parity, status);
   }
   out.flush(lane, logabs, phase, parity, status);
 }

@@ -55,3 +55,30 @@ def test_batch_equals_single_calls(cuda, lufqhe_mod, oracle, n):
     assert (np.abs(got["logabs"][ok] - la) / scale).max() < 1e-10
     d = np.abs(np.angle(np.exp(1j * (got["phase"][ok] - ph)))) / scale
     assert d.max() < 1e-10
+
+
+def test_plan_small_groups_equal_batched_calls(cuda, lufqhe_mod):
+    """A mixed plan's small pass: every n <= 16, group counts around a warp's
+    share and an item, padded rows, matrices left to refinement and FP64 and not
+    finite ones: the batched calls' bits."""
+    groups, want, off = [], [], 0
+    for n in range(1, 17):
+        rng = np.random.default_rng(n)
+        for count, pad in ((1, 0), (3, 1), (9, 0), (203, 0)):
+            L, _ = lufqhe_mod.gen_lll(count, n, seed=n + count)
+            A = cuda.zeros(count, n, n + pad, dtype=cuda.complex128, device="cuda")
+            A[:, :, :n] = L
+            if count == 9:
+                A[:8] = cuda.from_numpy(special(n, rng)).cuda()
+            groups.append((A, off))
+            off += count
+            want.append(results(lufqhe_mod.batch_lup_det(A, mode=lufqhe_mod.MODE_MIXED)))
+    out = lufqhe_mod.DetResult(*(cuda.zeros(off, dtype=d, device="cuda")
+                                 for d in (cuda.float64, cuda.float64, cuda.int8, cuda.int32)))
+    plan = lufqhe_mod.Plan(groups, out, autotune=False)
+    for _ in range(2):
+        plan.execute()
+    got = results(out)
+    for k in FIELDS:
+        assert np.array_equal(got[k], np.concatenate([w[k] for w in want]), equal_nan=True), k
+    plan.close()

@@ -280,7 +280,7 @@ __device__ void small_item(const WorkItem &w, unsigned char *base, int lane, flo
     load_rows(src, w.first + j, cnt * n, n, reinterpret_cast<double2 *>(HLw), Gd::LDH, NP, lane);
     __syncwarp();
     grid_unit<NP, LPM, NC, true, true>(src, w.first + j, w.out + j, cnt, n, HLw, Fw, Iw, lane, theta2,
-                                 w.share64k, refine, [](long long, bool) {}, out, logabs, phase,
+                                 w.share64k, refine, [](long long, bool, bool, const CFF &, int, int) {}, out, logabs, phase,
                                  parity, status);
   }
 }

@@ -17,7 +17,7 @@
 //  * Residual, solves, log det(I + E): lane (r, c) of the grid owns entries
 //    (GR a + r, GC b + c). R goes from the float-float accumulators straight
 //    into the solves' registers. The t loop of the residual is cut into blocks
-//    of TB steps whose slots are known at compile time, so that only the
+//    of 2, 4 or 8 steps whose slots are known at compile time, so that only the
 //    diagonal blocks carry masks.
 //  * Sums over a matrix (||E||_F, tr E, tr E^2) are taken in the order of a
 //    4 x 8 lane grid whatever the grid is, so the choice of grid changes no bit.
@@ -42,7 +42,6 @@ struct Grid {
   static constexpr int GR = LPM == 8 ? 2 : 4;
   static constexpr int GC = LPM / GR;
   static constexpr int SA = (NP + GR - 1) / GR, SB = (NP + GC - 1) / GC;
-  static constexpr int TB = GR;
   static constexpr int LDH = NP + 1;  // row stride of the double2 matrix and its hi/lo copy
   static constexpr int LDF = NP + 2;  // row stride of F: 16-byte rows for paired accesses
   // shared memory of one matrix: hi/lo copy, F, 2 NP ints. Where several
@@ -231,31 +230,107 @@ __device__ __forceinline__ bool lup_steps(float2 (&x)[NP], float2 *F, int n,
   }
 }
 
+// The LUP in shared memory on the 4 x 8 lane grid (one matrix per warp), rows
+// of F exchanged, rowat[i] the original row at position i.
+template <int NP, int NC>
+__device__ __forceinline__ bool lup_shared(float2 *F, int *rowat, int n, int lane, int &par) {
+  using Gd = Grid<NP, 32>;
+  constexpr int LDF = Gd::LDF, SA = Gd::SA, SB = Gd::SB;
+  constexpr bool GEN = NC == 0;
+  const int tr = lane >> 3, tc = lane & 7;
+  const float2 zero = make_float2(0.f, 0.f);
+#pragma unroll 1
+  for (int t = 0; t < n; ++t) {
+    const bool cand = lane >= t && lane < n;
+    unsigned mb = 0u;
+    float2 v = zero;
+    if (cand) {
+      v = F[lane * LDF + t];
+      mb = __float_as_uint(fabsf(v.x) + fabsf(v.y));
+    }
+    float best;
+    int bi;
+    if constexpr (GEN) {
+      const unsigned top = __reduce_max_sync(kFull, mb);
+      best = __uint_as_float(top);
+      bi = 31 - (int)__reduce_max_sync(kFull, (cand && mb == top) ? 31u - (unsigned)lane : 0u);
+    } else {
+      const unsigned key = __reduce_max_sync(kFull, cand ? ((mb & ~31u) | (31u - (unsigned)lane)) : 0u);
+      best = __uint_as_float(key & ~31u);
+      bi = 31 - (int)(key & 31u);
+    }
+    if (!(best > 0.0f) || !(best < INFINITY)) return false;  // zero/NaN/Inf pivot
+    // the pivot to all lanes, the multipliers by the lanes' (exchanged) rows
+    const float2 ut = shfl2(v, bi), vt = shfl2(v, t);
+    if (bi != t) {
+      if (lane < n && lane != t) {
+        const float2 a = F[bi * LDF + lane];
+        F[bi * LDF + lane] = F[t * LDF + lane];
+        F[t * LDF + lane] = a;
+      }
+      if (lane == t) {
+        F[t * LDF + t] = ut;
+        const int a = rowat[bi];
+        rowat[bi] = rowat[t];
+        rowat[t] = a;
+      }
+      if (lane == bi) v = vt;
+      par ^= 1;
+    }
+    const float2 rp = GEN ? crcpf(ut) : crcpf_approx(ut);
+    if (lane > t && lane < n) F[lane * LDF + t] = cmulf(v, rp);
+    __syncwarp();
+    float2 lv[SA], uv[SB];
+#pragma unroll
+    for (int a = 0; a < SA; ++a) {
+      const int i = 4 * a + tr;
+      lv[a] = (i > t && i < n) ? F[i * LDF + t] : zero;
+    }
+#pragma unroll
+    for (int b = 0; b < SB; ++b) {
+      const int k = 8 * b + tc;
+      uv[b] = (k > t && k < n) ? F[t * LDF + k] : zero;
+    }
+#pragma unroll
+    for (int a = 0; a < SA; ++a) {
+      if (4 * a + 3 <= t) continue;
+#pragma unroll
+      for (int b = 0; b < SB; ++b) {
+        if (8 * b + 7 <= t) continue;
+        const int i = 4 * a + tr, k = 8 * b + tc;
+        F[i * LDF + k] = cfms(F[i * LDF + k], lv[a], uv[b]);
+      }
+    }
+    __syncwarp();
+  }
+  return true;
+}
+
 // Residual steps of block TBLK (t in [TB TBLK, TB TBLK + TB), t < n): slots
 // whose rows or columns all lie before the block have nothing left to add.
-template <int NP, int LPM, int TBLK>
+template <int NP, int LPM, int TB, int TBLK>
 __device__ __forceinline__ void residual_block(float4 (&acc)[Grid<NP, LPM>::SA][Grid<NP, LPM>::SB],
                                                const float2 *F, int n, const GridLane<NP, LPM> &g) {
   using Gd = Grid<NP, LPM>;
-  constexpr int T0 = TBLK * Gd::TB;
+  constexpr int T0 = TBLK * TB;
   if constexpr (T0 < NP) {
     if (T0 >= n) return;
 #pragma unroll 1
-    for (int t = T0; t < min(T0 + Gd::TB, n); ++t) {
+    for (int t = T0; t < min(T0 + TB, n); ++t) {
       float2 Uv[Gd::SB];
 #pragma unroll
       for (int b = 0; b < Gd::SB; ++b) {
         if (Gd::GC * b + Gd::GC <= T0) continue;
         const int k = Gd::GC * b + g.c;
         Uv[b] = F[t * Gd::LDF + k];
-        if (Gd::GC * b < T0 + Gd::TB && k < t) Uv[b] = make_float2(0.f, 0.f);
+        if (Gd::GC * b < T0 + TB && k < t) Uv[b] = make_float2(0.f, 0.f);
       }
 #pragma unroll
       for (int a = 0; a < Gd::SA; ++a) {
         if (Gd::GR * a + Gd::GR <= T0) continue;
         const int i = Gd::GR * a + g.r;
         float2 l = F[i * Gd::LDF + t];
-        if (Gd::GR * a < T0 + Gd::TB) {
+        if (Gd::GR * a < T0 + TB) {
           if (i < t) l = make_float2(0.f, 0.f);
           if (i == t) l = make_float2(1.f, 0.f);
         }
@@ -266,7 +341,7 @@ __device__ __forceinline__ void residual_block(float4 (&acc)[Grid<NP, LPM>::SA][
         }
       }
     }
-    residual_block<NP, LPM, TBLK + 1>(acc, F, n, g);
+    residual_block<NP, LPM, TB, TBLK + 1>(acc, F, n, g);
   }
 }
 
@@ -276,12 +351,12 @@ __device__ __forceinline__ void residual_block(float4 (&acc)[Grid<NP, LPM>::SA][
 // rule or 0 for the generic one. The outcome is uniform over the group:
 //  TILE_ACCEPT: prod, exp_sum, corr, par hold the determinant;
 //  TILE_REFINE (NC != 0): ||E||_F within theta but above the FP32 solves' cap;
-//    F holds L\U in pivoted order and, with KEEP_Y, HL's float2 view (row
-//    stride n + 1) Y = L^-1 R;
+//    F holds L\U in pivoted order and HL's float2 view (row stride n + 1)
+//    Y = L^-1 R;
 //  TILE_REJECT, TILE_NONFINITE: for the FP64 route, or not finite.
 // Lanes of a group past the batch's end run on whatever the group holds; every
 // address depends on n and the lane only, or on positions below 32.
-template <int NP, int LPM, int NC, bool KEEP_Y>
+template <int NP, int LPM, int NC>
 __device__ __forceinline__ int grid_factor(float4 *HL, float2 *F, int *ints, const int n_rt,
                                            int lane, float theta2, CFF &prod, int &exp_sum,
                                            float2 &corr, int &par) {
@@ -289,6 +364,13 @@ __device__ __forceinline__ int grid_factor(float4 *HL, float2 *F, int *ints, con
   constexpr int GR = Gd::GR, GC = Gd::GC, SA = Gd::SA, SB = Gd::SB;
   constexpr int LDH = Gd::LDH, LDF = Gd::LDF;
   constexpr bool GEN = NC == 0;
+  // n = 17..24: the LUP in shared memory and wider residual blocks, whose code
+  // is half the size (32768 LLL x n=24, FP32 pass, us: 921 in registers, 825 in
+  // shared memory, 767 with blocks of 8; Gaussian 680, 697, 670). n = 32 is
+  // faster in registers (8192 LLL 412 against 492 to 547), the padded sizes
+  // above 24 in registers with blocks of 8.
+  constexpr bool kShared = NP == 24;
+  constexpr int kTB = NP == 24 || (NP == 32 && GEN) ? 8 : Gd::GR;
   const int n = GEN ? n_rt : NC;
   const GridLane<NP, LPM> g(lane);
   const int sub = g.sub, r = g.r, c = g.c;
@@ -340,6 +422,7 @@ __device__ __forceinline__ int grid_factor(float4 *HL, float2 *F, int *ints, con
       split_words(v.x, adj, xh, xl);
       split_words(v.y, adj, yh, yl);
       HL[idx] = make_float4(xh, yh, xl, yl);
+      if constexpr (kShared) F[i * LDF + k] = make_float2(xh, yh);
       i += di;
       k += dk;
       if (k >= n) {
@@ -353,7 +436,19 @@ __device__ __forceinline__ int grid_factor(float4 *HL, float2 *F, int *ints, con
   // 3. FP32 LUP: lane = row
   bool fail = false;
   par = 0;
-  {
+  if constexpr (kShared) {
+    int *rowat = ints;  // (the exponents are done with)
+    if (sub < NP) rowat[sub] = sub;
+    if constexpr (NC < NP) {
+      // padding: rows and columns past n are zero
+      for (int e = lane; e < NP * NP; e += 32) {
+        const int i = e / NP, k = e - i * NP;
+        if (i >= n || k >= n) F[i * LDF + k] = zero;
+      }
+    }
+    __syncwarp();
+    if (!lup_shared<NP, NC>(F, rowat, n, lane, par)) return TILE_REJECT;
+  } else {
     float2 x[NP];
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
@@ -398,7 +493,7 @@ __device__ __forceinline__ int grid_factor(float4 *HL, float2 *F, int *ints, con
                         : make_float4(0.f, 0.f, 0.f, 0.f);
       }
     }
-    residual_block<NP, LPM, 0>(acc, F, n, g);
+    residual_block<NP, LPM, kTB, 0>(acc, F, n, g);
 #pragma unroll
     for (int a = 0; a < SA; ++a)
 #pragma unroll
@@ -438,7 +533,7 @@ __device__ __forceinline__ int grid_factor(float4 *HL, float2 *F, int *ints, con
       }
     }
   }
-  if constexpr (KEEP_Y && !GEN) {
+  if constexpr (!GEN) {
 #pragma unroll
     for (int a = 0; a < SA; ++a)
 #pragma unroll
@@ -661,8 +756,8 @@ __device__ __noinline__ void grid_refactor_call(const Src src, long long sb, int
 // The `cnt` matrices from b0 of src, staged in the warp's area (group q at
 // HLw + q kHL), into outputs ob0 ..: the FP32 path, then what it does not accept:
 // refined or refactorised right here (INPLACE, n <= 16), or handed to
-// defer(b, routed). share64k: the share routed straight to FP64. CALL: FP64 out
-// of line.
+// defer(b, routed, can_refine, prod, exp_sum, par). share64k: the share routed
+// straight to FP64. CALL: FP64 out of line.
 template <int NP, int LPM, int NC, bool INPLACE, bool CALL, class Src, class Defer>
 __device__ __forceinline__ void grid_unit(const Src &src, long long b0, long long ob0, int cnt,
                                           int n, float4 *HLw, float2 *Fw, int *Iw, int lane,
@@ -674,7 +769,7 @@ __device__ __forceinline__ void grid_unit(const Src &src, long long b0, long lon
   CFF prod;
   int exp_sum, par;
   float2 corr;
-  int code = grid_factor<NP, LPM, NC, INPLACE>(HLw + grp * Gd::kHL, Fw + grp * Gd::kF,
+  int code = grid_factor<NP, LPM, NC>(HLw + grp * Gd::kHL, Fw + grp * Gd::kF,
                                                Iw + grp * 2 * NP, n, lane, theta2, prod, exp_sum,
                                                corr, par);
   bool routed = false;
@@ -685,11 +780,16 @@ __device__ __forceinline__ void grid_unit(const Src &src, long long b0, long lon
 #pragma unroll 1
   for (int q = 0; q < cnt; ++q) {
     const int from = q * LPM;
-    const int cq = __shfl_sync(kFull, code, from);
-    const CFF pq = shfl_cff(prod, from, false);
-    const int eq = __shfl_sync(kFull, exp_sum, from);
-    const int rq = __shfl_sync(kFull, par, from);
-    float2 kq = shfl2(corr, from);
+    int cq = code, eq = exp_sum, rq = par;
+    CFF pq = prod;
+    float2 kq = corr;
+    if constexpr (Gd::G > 1) {
+      cq = __shfl_sync(kFull, code, from);
+      pq = shfl_cff(prod, from, false);
+      eq = __shfl_sync(kFull, exp_sum, from);
+      rq = __shfl_sync(kFull, par, from);
+      kq = shfl2(corr, from);
+    }
     const long long ob = ob0 + q;
     if (cq == TILE_ACCEPT) {
       out.push(lane, ob, pq, eq, kq, rq, logabs, phase, parity, status);
@@ -699,9 +799,9 @@ __device__ __forceinline__ void grid_unit(const Src &src, long long b0, long lon
       emit_nonfinite(lane, ob, logabs, phase, parity, status);
       continue;
     }
-    const bool rt = __shfl_sync(kFull, (int)routed, from) != 0;
+    const bool rt = Gd::G > 1 ? __shfl_sync(kFull, (int)routed, from) != 0 : routed;
     if constexpr (!INPLACE) {
-      defer(b0 + q, rt);
+      defer(b0 + q, rt, cq == TILE_REFINE && refine, pq, eq, rq);
     } else {
       float4 *HLq = HLw + q * Gd::kHL;
       float2 *Fq = Fw + q * Gd::kF;

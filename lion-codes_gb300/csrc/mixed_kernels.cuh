@@ -119,7 +119,10 @@ constexpr int kDeferMinN = 24;
 // The same of the lane-grid kernels: shared memory holds 16 warps an SM at
 // NP = 16 (13.5 KB each), 15 at 24 (14.8 KB) and 8 at 32 (25.7 KB).
 constexpr int grid_warps(int np) { return np == 24 ? 3 : 4; }
-constexpr int grid_min_ctas(int np) { return np == 24 ? 5 : np == 32 ? 2 : 4; }
+// (n = 32 itself is compiled for 3 CTAs although 2 fit: with 168 registers instead
+// of 255 the compiler moves less code ahead of its use, 412 us instead of 557
+// for 8192 LLL matrices; the padded sizes gain from the 255.)
+constexpr int grid_min_ctas(int np, int nc) { return np == 24 ? 5 : np == 32 ? (nc ? 3 : 2) : 4; }
 // Warps of the FP64 pass's CTA (one CTA per SM).
 constexpr int kFallbackMaxWarps = 20;
 // Warps of a CTA of the correction pass after the finish kernel.
@@ -167,11 +170,12 @@ constexpr int fac_copies() {
   return std::is_same<Src, DenseSource>::value ? 0 : 1;
 }
 
-// Save a TILE_REFINE matrix; false (warp-uniform) if the buffer is full.
+// Save a TILE_REFINE matrix (F at row stride ldf); false (warp-uniform) if the
+// buffer is full.
 template <int N>
-__device__ bool save_refine(CallHead *head, unsigned char *buf, long long cap, long long b,
-                            const float2 *F, const float2 *Rm, const CFF &prod, int exp_sum,
-                            int par, int lane) {
+__device__ __noinline__ bool save_refine(CallHead *head, unsigned char *buf, long long cap, long long b,
+                            const float2 *F, int ldf, const float2 *Rm, const CFF &prod,
+                            int exp_sum, int par, int lane) {
   constexpr int NL = N * (N + 1);
   unsigned long long k = 0;
   if (lane == 0) k = atomicAdd(&head->refine_saved, 1ull);
@@ -181,7 +185,7 @@ __device__ bool save_refine(CallHead *head, unsigned char *buf, long long cap, l
   float2 *dF = reinterpret_cast<float2 *>(e + sizeof(RefineHead));
   float2 *dY = dF + NL;
   for (int q = lane; q < NL; q += 32) {
-    dF[q] = F[q];
+    dF[q] = F[q + q / (N + 1) * (ldf - (N + 1))];
     dY[q] = Rm[q];
   }
   if (lane == 0) {
@@ -254,13 +258,15 @@ __global__ void __launch_bounds__(kMaxWarpsMixed * 32)
 
 // The FP32 pass of the lane-grid path: each warp takes Grid::G consecutive
 // matrices at a time. NC = n for the register-tiled sizes, 0 for the generic
-// rule. DEFER: rejected matrices go to the call's pending list; else they are
-// refined or refactorised in FP64 right away, one at a time by the whole warp.
+// rule. DEFER: rejected matrices go to the call's pending list and (n = 24, 32)
+// the ones to refine to the saved matrices; else they are refined or
+// refactorised in FP64 right away, one at a time by the whole warp.
 template <int NP, int LPM, int NC, bool DEFER, class Src>
-__global__ void __launch_bounds__(grid_warps(NP) * 32, grid_min_ctas(NP))
+__global__ void __launch_bounds__(grid_warps(NP) * 32, grid_min_ctas(NP, NC))
     lup_mixed_grid_kernel(Src src, int n_rt, long long batch, float theta2,
                           unsigned int share64k, CallHead *head, unsigned int *pend, int refine,
-                          int bulk, double *__restrict__ logabs, double *__restrict__ phase,
+                          unsigned char *saved, long long saved_cap, int bulk,
+                          double *__restrict__ logabs, double *__restrict__ phase,
                           int8_t *__restrict__ parity, int32_t *__restrict__ status) {
   using Gd = Grid<NP, LPM>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -303,32 +309,37 @@ __global__ void __launch_bounds__(grid_warps(NP) * 32, grid_min_ctas(NP))
     }
     if (!staged) load_rows(src, b0, cnt * n, n, M, Gd::LDH, NP, lane);
     __syncwarp();
+    // DEFER: a matrix within theta but above the FP32 solves' cap gets its back
+    // substitution refined by the next pass, if the buffer has room; the others
+    // are listed for FP64
     grid_unit<NP, LPM, NC, !DEFER, false>(
         src, b0, b0, cnt, n, HLw, Fw, Iw, lane, theta2, share64k, refine != 0,
-        [&](long long b, bool routed) { defer_fp64(head, pend, b, lane, routed); }, out, logabs,
-        phase, parity, status);
+        [&](long long b, bool routed, bool can_refine, const CFF &prod, int exp_sum, int par) {
+          if constexpr (NC != 0)
+            if (can_refine && saved &&
+                save_refine<NC>(head, saved, saved_cap, b, Fw, Gd::LDF,
+                                reinterpret_cast<const float2 *>(HLw), prod, exp_sum, par, lane))
+              return;
+          defer_fp64(head, pend, b, lane, routed);
+        },
+        out, logabs, phase, parity, status);
   }
   out.flush(lane, logabs, phase, parity, status);
 }
 
 
-template <int N, class Src, bool INPLACE = false>
+// n = 24 and 32, a batch in mapped host memory: the FP32 path with everything
+// else in place (the kernel waits on the link and has compute to spare), except
+// the corrections of its FP64 refactorisations, which are listed for a pass of
+// their own.
+template <int N>
 __global__ void __launch_bounds__(tile_max_warps(N) * 32, tile_min_ctas(N))
-    lup_mixed_tile_kernel(Src src, long long batch, float theta2,
-                          unsigned int share64k, CallHead *head, unsigned int *pend,
-                          double2 *spill, unsigned char *refine, long long refine_cap,
-                          unsigned char *corr_list, long long corr_cap, int bulk,
-                          double *__restrict__ logabs,
+    lup_mixed_tile_kernel(DenseSource src, long long batch, float theta2, unsigned int share64k,
+                          CallHead *head, double2 *spill, int refine, unsigned char *corr_list,
+                          long long corr_cap, double *__restrict__ logabs,
                           double *__restrict__ phase, int8_t *__restrict__ parity,
                           int32_t *__restrict__ status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  // every FP64 factorisation goes to the FP64 pass, so this kernel carries no
-  // FP64 factorisation code (a smaller instruction footprint). INPLACE keeps
-  // them in this kernel: for a batch read over the host link, where the FP32
-  // pass waits on the link and has compute to spare.
-  constexpr bool DEFER = !INPLACE;
-  // complex128 device batches: the matrix is staged by bulk copies (bulk != 0)
-  constexpr bool BULK = !INPLACE && std::is_same<Src, DenseSource>::value;
   constexpr int LDS = N + 1;
   constexpr size_t NL = (size_t)N * LDS;
   const int warps = blockDim.x >> 5;
@@ -344,49 +355,27 @@ __global__ void __launch_bounds__(tile_max_warps(N) * 32, tile_min_ctas(N))
   int *er = reinterpret_cast<int *>(base) + warp * 2 * N;
   int *ec = er + N;
   const CorrScratch cs{F, er, hold};
-  // INPLACE: this warp's copy of its current matrix in global memory (a few
-  // KB per warp, so the copies stay in L2); an FP64 refactorisation reloads
-  // it from there instead of reading the matrix over the host link again
-  double2 *own = INPLACE ? spill + ((size_t)blockIdx.x * warps + warp) * N * N : nullptr;
-  __shared__ __align__(8) uint64_t bars[kMaxWarpsMixed];
-  WarpBulk wb;
-  if constexpr (BULK)
-    if (bulk) wb.init(&bars[warp], lane);
+  // this warp's copy of its current matrix in global memory (a few KB per warp,
+  // so the copies stay in L2); an FP64 refactorisation reloads it from there
+  // instead of reading the matrix over the host link again
+  double2 *own = spill + ((size_t)blockIdx.x * warps + warp) * N * N;
 
   DeferredOut out;
-  // the next matrix is claimed one ahead, so that its bytes can be on their
-  // way to L2 while the current one is factorised
   long long b = claim_matrix(head, lane, -1);
   long long nb = b < batch ? claim_matrix(head, lane, b) : batch;
   for (; b < batch; b = nb, nb = b < batch ? claim_matrix(head, lane, b) : batch) {
     __syncwarp();
     double2 *M = reinterpret_cast<double2 *>(HL);
-    if constexpr (BULK)
-      if (bulk && nb < batch && lane == 0)
-        prefetch_matrix_l2(src.A + (size_t)nb * N * src.lda, N, src.lda);
     if (share64k && route_fp64_entry(src.first(b, N), share64k)) {
-      if constexpr (DEFER)
-        defer_fp64(head, pend, b, lane, true);
-      else
-        fallback_fp64_src(src, b, N, M, LDS, hold, lane, b, logabs, phase, parity, status,
-                          LUFQHE_ST_FP64, &cs);
+      fallback_fp64_src(src, b, N, M, LDS, hold, lane, b, logabs, phase, parity, status,
+                        LUFQHE_ST_FP64, &cs);
       continue;
     }
-    bool staged = false;
-    if constexpr (BULK) {
-      if (bulk && !wb.broken) {
-        if (!wb.load(src.A + (size_t)b * N * src.lda, N, src.lda, M, LDS, lane)) {
-          emit_wait_timeout(lane, b, logabs, phase, parity, status);
-          continue;
-        }
-        staged = true;  // finite check: in the exponent pass
-      }
-    }
-    if (!staged && src.load(b, N, M, LDS, lane)) {
+    if (src.load(b, N, M, LDS, lane)) {
       emit_nonfinite(lane, b, logabs, phase, parity, status);
       continue;
     }
-    if constexpr (INPLACE) {
+    {
       BlockWalk w(lane, N);
       for (int e = lane; e < N * N; e += 32) {
         own[e] = M[w.i * LDS + w.k];
@@ -396,50 +385,29 @@ __global__ void __launch_bounds__(tile_max_warps(N) * 32, tile_min_ctas(N))
     CFF prod;
     int exp_sum, par;
     float2 corr;
-    if constexpr (DEFER) {
-      const int code =
-          mixed_factor_tile_ex<N, true>(HL, F, er, ec, lane, theta2, prod, exp_sum, corr, par);
-      if (code == TILE_ACCEPT)
-        out.push(lane, b, prod, exp_sum, corr, par, logabs, phase, parity, status);
-      else if (code == TILE_NONFINITE)
-        emit_nonfinite(lane, b, logabs, phase, parity, status);
-      // a matrix within theta but above the FP32 solves' cap gets its back
-      // substitution refined in the next pass, if the buffer has room
-      else if (!(code == TILE_REFINE && refine &&
-                 save_refine<N>(head, refine, refine_cap, b, F,
-                                reinterpret_cast<const float2 *>(HL), prod, exp_sum, par, lane)))
-        defer_fp64(head, pend, b, lane, false);
+    const int code =
+        mixed_factor_tile_ex<N, true>(HL, F, er, ec, lane, theta2, prod, exp_sum, corr, par);
+    if (code == TILE_ACCEPT ||
+        (code == TILE_REFINE && refine &&
+         mixed_refine_tile<N>(F, reinterpret_cast<float2 *>(HL),
+                              reinterpret_cast<float2 *>(HL) + N * (N + 1),
+                              reinterpret_cast<float2 *>(er), lane, theta2,
+                              tile_la_est(prod, exp_sum), corr))) {
+      out.push(lane, b, prod, exp_sum, corr, par, logabs, phase, parity, status);
     } else {
-      // in place: the refinement (refine_cap != 0), then FP64 (the host-link
-      // variant, which has compute to spare)
-      const int code =
-          mixed_factor_tile_ex<N, true>(HL, F, er, ec, lane, theta2, prod, exp_sum, corr, par);
-      if (code == TILE_NONFINITE) {
-        emit_nonfinite(lane, b, logabs, phase, parity, status);
-        continue;
-      }
-      if (code == TILE_ACCEPT ||
-          (code == TILE_REFINE && refine_cap != 0 &&
-           mixed_refine_tile<N>(F, reinterpret_cast<float2 *>(HL),
-                                reinterpret_cast<float2 *>(HL) + N * (N + 1),
-                                reinterpret_cast<float2 *>(er), lane, theta2,
-                                tile_la_est(prod, exp_sum), corr))) {
-        out.push(lane, b, prod, exp_sum, corr, par, logabs, phase, parity, status);
-      } else {
-        // the factors (and the warp's copy of the matrix) are listed for the
-        // correction pass, so that no warp stops reading the link for one
-        const FacList fl{&head->corr_count, corr_list, corr_cap, 1};
-        fallback_fp64_src<DenseSource, true>(DenseSource{own, N}, 0, N, M, LDS, hold, lane, b,
-                                             logabs, phase, parity, status, LUFQHE_ST_FALLBACK,
-                                             &cs, corr_list != nullptr ? &fl : nullptr);
-      }
+      // the factors (and the warp's copy of the matrix) are listed for the
+      // correction pass, so that no warp stops reading the link for one
+      const FacList fl{&head->corr_count, corr_list, corr_cap, 1};
+      fallback_fp64_src<DenseSource, true>(DenseSource{own, N}, 0, N, M, LDS, hold, lane, b,
+                                           logabs, phase, parity, status, LUFQHE_ST_FALLBACK,
+                                           &cs, &fl);
     }
   }
   out.flush(lane, logabs, phase, parity, status);
 }
 
-// The passes after the FP32 pass, as one kernel in the FP32 pass's
-// shared-memory layout (n >= 24): the FP64 refactorisations of the matrices
+// The passes after the FP32 pass, as one kernel in the tile path's
+// shared-memory layout (n = 24, 32): the FP64 refactorisations of the matrices
 // the FP32 pass rejected, dealt out at a fixed stride over the grid's warps
 // first, while the warps without one refine the saved matrices (claimed one at
 // a time; a refinement that fails is refactorised in FP64 on the spot). The
@@ -728,104 +696,108 @@ int launch_fac_correct(Src src, const CallHead *head, const unsigned char *list,
   return check_cuda(cudaGetLastError(), "lup_mixed_fac_correct_kernel launch");
 }
 
-template <int N, class Src>
-int launch_mixed_tile(Src src, long long batch, float theta2, double *logabs, double *phase,
-                      int8_t *parity, int32_t *status, cudaStream_t stream, bool inplace) {
-  // only dense batches of the deferring sizes have an in-place variant
-  constexpr bool kHasInplace = N >= kDeferMinN && std::is_same<Src, DenseSource>::value;
-  if (!kHasInplace) inplace = false;
-  const size_t per_warp = tile_smem_per_warp<N>();
-  // small CTAs: the register-heavy residual tile limits residency, and
-  // smaller CTAs let the scheduler fill an SM with several of them
-  int warps = (int)(device_smem_optin() / per_warp);
-  int wcap = tile_max_warps(N);
-  if (g_tile_warps > 0 && g_tile_warps < wcap) wcap = g_tile_warps;
-  if (warps > wcap) warps = wcap;
-  const size_t smem = per_warp * warps;
-  auto kern = lup_mixed_tile_kernel<N, Src, false>;
-  if constexpr (kHasInplace)
-    if (inplace) kern = lup_mixed_tile_kernel<N, Src, true>;
+// Shared-memory limit, and the grid of `warps`-warp CTAs over `units` units.
+template <class K>
+int grid_geometry(K kern, int warps, size_t smem, long long units, int *grid) {
   int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)smem),
-                      "cudaFuncSetAttribute(mixed tile)");
+                      "cudaFuncSetAttribute(mixed)");
   if (rc) return rc;
   int per_sm = 0;
   rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, smem),
-                  "occupancy(mixed tile)");
+                  "occupancy(mixed)");
   if (rc) return rc;
-  if (per_sm < 1) per_sm = 1;
-  long long want = (batch + warps - 1) / warps;
-  long long cap = (long long)device_sm_count() * per_sm;
-  int grid = (int)(want < cap ? want : cap);
-  // n >= 24 from device memory: the refinements and FP64 refactorisations go
-  // to the finish kernel through the call's pending list and saved matrices
-  const bool two_pass = !inplace;
-  long long refine_cap = 0;
-  size_t refine_bytes = 0;
-  if (two_pass && g_mixed_refine) {
-    refine_cap = std::max<long long>(256, (long long)(kRefineShare * (double)batch));
-    refine_cap = std::min<long long>(refine_cap, batch);
-    refine_bytes = (size_t)refine_cap * refine_entry_bytes<N>();
-  }
-  const size_t spill_bytes = inplace ? (size_t)grid * warps * N * N * sizeof(double2) : 0;
-  // the host-link variant's correction list (sizes with a corrected FP64 route)
-  long long corr_cap = 0;
-  if (inplace && N >= kCorrectMinN) {
-    corr_cap = std::max<long long>(256, (long long)(kCorrShare * (double)batch));
-    corr_cap = std::min<long long>(corr_cap, batch);
-  }
-  // the device path's list of FP64 factors for the correction pass (an
-  // overflow is corrected in the finish kernel itself)
-  long long fac_cap = 0;
-  if (two_pass && N >= kCorrectMinN && N <= kCorrectMaxN) {
-    fac_cap = std::max<long long>(256, (long long)(kCorrShare * (double)batch));
-    fac_cap = std::min<long long>(fac_cap, batch);
-  }
+  const long long want = (units + warps - 1) / warps;
+  const long long cap = (long long)device_sm_count() * std::max(1, per_sm);
+  *grid = (int)std::min(want, cap);
+  return LUFQHE_SUCCESS;
+}
+
+// Warps per CTA of the in-place and finish kernels, in the tile layout.
+template <int N>
+int tile_warps() {
+  int warps = (int)(device_smem_optin() / tile_smem_per_warp<N>());
+  int cap = tile_max_warps(N);
+  if (g_tile_warps > 0 && g_tile_warps < cap) cap = g_tile_warps;
+  return std::min(warps, cap);
+}
+// Room for `share` of a batch.
+inline long long share_cap(double share, long long batch) {
+  return std::min(batch, std::max<long long>(256, (long long)(share * (double)batch)));
+}
+
+// n = 24 and 32, a batch read over the host link: one kernel, then the
+// corrections of its FP64 refactorisations.
+template <int N>
+int launch_mixed_hostlink(DenseSource src, long long batch, float theta2, double *logabs,
+                          double *phase, int8_t *parity, int32_t *status, cudaStream_t stream) {
+  auto kern = lup_mixed_tile_kernel<N>;
+  const int warps = tile_warps<N>();
+  const size_t smem = tile_smem_per_warp<N>() * warps;
+  int grid = 0;
+  int rc = grid_geometry(kern, warps, smem, batch, &grid);
+  if (rc) return rc;
+  const long long corr_cap = share_cap(kCorrShare, batch);
   CallState cs;
-  if (two_pass || inplace || needs_counter(batch, (long long)grid * warps)) {
-    rc = cs.acquire(two_pass ? (size_t)batch : 0, refine_bytes, spill_bytes, stream,
-                    inplace ? (size_t)corr_cap * (size_t)fac_entry_bytes(N, true)
-                            : (size_t)fac_cap * (size_t)fac_entry_bytes(N, fac_copies<Src>()));
-    if (rc) return cs.release(stream, rc);
-  }
-  // in-place kernels: refine_cap says whether the refinement is on
-  if (!two_pass) refine_cap = g_mixed_refine;
+  rc = cs.acquire(0, 0, (size_t)grid * warps * N * N * sizeof(double2), stream,
+                  (size_t)corr_cap * (size_t)fac_entry_bytes(N, true));
+  if (rc) return cs.release(stream, rc);
   {
-    KernelTimer timer(inplace ? "lup_mixed_tile_kernel_hostlink" : "lup_mixed_tile_kernel", N,
-                      stream);
-    kern<<<grid, warps * 32, smem, stream>>>(src, batch, theta2, fp64_share_64k(N), cs.head, cs.pend,
-                                             cs.spill, cs.refine, refine_cap, cs.corr, corr_cap,
-                                             bulk_for(src), logabs, phase, parity, status);
+    KernelTimer timer("lup_mixed_tile_kernel_hostlink", N, stream);
+    kern<<<grid, warps * 32, smem, stream>>>(src, batch, theta2, fp64_share_64k(N), cs.head,
+                                             cs.spill, g_mixed_refine, cs.corr, corr_cap, logabs,
+                                             phase, parity, status);
     timer.stop();
   }
   rc = check_cuda(cudaGetLastError(), "lup_mixed_tile_kernel launch");
-  if (!rc && corr_cap > 0) {
-    if constexpr (kHasInplace && N >= kCorrectMinN && N <= kCorrectMaxN)
-      rc = launch_fac_correct<N, Src, true>(src, cs.head, cs.corr, corr_cap, logabs, phase,
-                                            parity, status, stream);
+  if (!rc)
+    rc = launch_fac_correct<N, DenseSource, true>(src, cs.head, cs.corr, corr_cap, logabs, phase,
+                                                  parity, status, stream);
+  return cs.release(stream, rc);
+}
+
+// n = 24 and 32: the FP32 pass on the lane grid; the refinements and the FP64
+// refactorisations it leaves, side by side in one kernel; the corrections of
+// those refactorisations, each by a whole CTA.
+template <int N, class Src>
+int launch_mixed_tile(Src src, long long batch, float theta2, double *logabs, double *phase,
+                      int8_t *parity, int32_t *status, cudaStream_t stream) {
+  using Gd = Grid<N, 32>;
+  auto kern = lup_mixed_grid_kernel<N, 32, N, true, Src>;
+  auto fk = lup_mixed_finish_kernel<N, Src>;
+  constexpr int gwarps = grid_warps(N);
+  const size_t gsmem = Gd::kWarpBytes * gwarps;
+  const int fwarps = tile_warps<N>();
+  const size_t fsmem = tile_smem_per_warp<N>() * fwarps;
+  int grid = 0, fgrid = 0;
+  int rc = grid_geometry(kern, gwarps, gsmem, batch, &grid);
+  if (!rc) rc = grid_geometry(fk, fwarps, fsmem, batch, &fgrid);
+  if (rc) return rc;
+  const long long refine_cap = g_mixed_refine ? share_cap(kRefineShare, batch) : 0;
+  // the list of FP64 factors (an overflow is corrected in the finish kernel)
+  const long long fac_cap = share_cap(kCorrShare, batch);
+  CallState cs;
+  rc = cs.acquire((size_t)batch, (size_t)refine_cap * refine_entry_bytes<N>(), 0, stream,
+                  (size_t)fac_cap * (size_t)fac_entry_bytes(N, fac_copies<Src>()));
+  if (rc) return cs.release(stream, rc);
+  {
+    KernelTimer timer("lup_mixed_tile_kernel", N, stream);
+    kern<<<grid, gwarps * 32, gsmem, stream>>>(src, N, batch, theta2, fp64_share_64k(N), cs.head,
+                                               cs.pend, g_mixed_refine, cs.refine, refine_cap,
+                                               bulk_for(src), logabs, phase, parity, status);
+    timer.stop();
   }
-  // the refinements and the FP64 refactorisations, side by side in one kernel,
-  // then the corrections of those refactorisations, each by a whole CTA
-  if (!rc && two_pass) {
-    if constexpr (N >= kDeferMinN) {
-      auto fk = lup_mixed_finish_kernel<N, Src>;
-      rc = check_cuda(cudaFuncSetAttribute(fk, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem),
-                      "cudaFuncSetAttribute(mixed finish)");
-      if (!rc) {
-        KernelTimer timer("lup_mixed_finish_kernel", N, stream);
-        fk<<<grid, warps * 32, smem, stream>>>(src, cs.head, cs.pend, cs.refine, refine_cap,
-                                               theta2, cs.corr, fac_cap, logabs, phase, parity,
-                                               status);
-        timer.stop();
-        rc = check_cuda(cudaGetLastError(), "lup_mixed_finish_kernel launch");
-      }
-      if (!rc && fac_cap > 0)
-        rc = launch_fac_correct<N, Src, fac_copies<Src>() != 0>(src, cs.head, cs.corr, fac_cap,
-                                                                logabs, phase, parity, status,
-                                                                stream);
-    }
+  rc = check_cuda(cudaGetLastError(), "lup_mixed_grid_kernel launch");
+  if (!rc) {
+    KernelTimer timer("lup_mixed_finish_kernel", N, stream);
+    fk<<<fgrid, fwarps * 32, fsmem, stream>>>(src, cs.head, cs.pend, cs.refine, refine_cap, theta2,
+                                              cs.corr, fac_cap, logabs, phase, parity, status);
+    timer.stop();
+    rc = check_cuda(cudaGetLastError(), "lup_mixed_finish_kernel launch");
   }
+  if (!rc)
+    rc = launch_fac_correct<N, Src, fac_copies<Src>() != 0>(src, cs.head, cs.corr, fac_cap, logabs,
+                                                            phase, parity, status, stream);
   return cs.release(stream, rc);
 }
 
@@ -836,29 +808,21 @@ int launch_mixed_grid(Src src, int n, long long batch, float theta2, double *log
   auto kern = lup_mixed_grid_kernel<NP, LPM, NC, DEFER, Src>;
   constexpr int warps = grid_warps(NP);
   const size_t smem = Gd::kWarpBytes * warps;
-  int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem),
-                      "cudaFuncSetAttribute(mixed grid)");
-  if (rc) return rc;
-  int per_sm = 0;
-  rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, smem),
-                  "occupancy(mixed grid)");
-  if (rc) return rc;
-  if (per_sm < 1) per_sm = 1;
   const long long units = (batch + Gd::G - 1) / Gd::G;
-  const long long want = (units + warps - 1) / warps;
-  const long long cap = (long long)device_sm_count() * per_sm;
-  const int grid = (int)(want < cap ? want : cap);
+  int grid = 0;
+  int rc = grid_geometry(kern, warps, smem, units, &grid);
+  if (rc) return rc;
   CallState cs;
   if (DEFER || needs_counter(units, (long long)grid * warps)) {
     rc = cs.acquire(DEFER ? (size_t)batch : 0, 0, 0, stream);
     if (rc) return cs.release(stream, rc);
   }
   {
-    KernelTimer timer("lup_mixed_grid_kernel", n, stream);
+    // (recorded under the names of the two rules)
+    KernelTimer timer(NC ? "lup_mixed_tile_kernel" : "lup_mixed_kernel", n, stream);
     kern<<<grid, warps * 32, smem, stream>>>(src, n, batch, theta2, fp64_share_64k(n), cs.head,
-                                             cs.pend, g_mixed_refine, bulk_for(src), logabs,
-                                             phase, parity, status);
+                                             cs.pend, g_mixed_refine, nullptr, 0, bulk_for(src),
+                                             logabs, phase, parity, status);
     timer.stop();
   }
   rc = check_cuda(cudaGetLastError(), "lup_mixed_grid_kernel launch");
@@ -906,8 +870,14 @@ int launch_mixed_src(Src src, int n, long long batch, double *logabs, double *ph
       case 8: return launch_mixed_small<8, 8, 8>(src, n, batch, th2, logabs, phase, parity, status, stream);
       case 12: return launch_mixed_small<12, 16, 12>(src, n, batch, th2, logabs, phase, parity, status, stream);
       case 16: return launch_mixed_small<16, 16, 16>(src, n, batch, th2, logabs, phase, parity, status, stream);
-      case 24: return launch_mixed_tile<24>(src, batch, th2, logabs, phase, parity, status, stream, inplace);
-      case 32: return launch_mixed_tile<32>(src, batch, th2, logabs, phase, parity, status, stream, inplace);
+      case 24:
+        if constexpr (std::is_same<Src, DenseSource>::value)
+          if (inplace) return launch_mixed_hostlink<24>(src, batch, th2, logabs, phase, parity, status, stream);
+        return launch_mixed_tile<24>(src, batch, th2, logabs, phase, parity, status, stream);
+      case 32:
+        if constexpr (std::is_same<Src, DenseSource>::value)
+          if (inplace) return launch_mixed_hostlink<32>(src, batch, th2, logabs, phase, parity, status, stream);
+        return launch_mixed_tile<32>(src, batch, th2, logabs, phase, parity, status, stream);
       default: break;
     }
   }

@@ -63,13 +63,26 @@ __device__ __forceinline__ int exp_field_c(double2 v) { return max(exp_field(v.x
 // units, 2^-45 of a typical |R_ij|. T is the top-bit position of the entry's
 // largest term, found by an exponent pass first.
 //
-// acc += (-1)^neg (m1 m2 >> r) mod 2^64, r >= 0 (m1, m2 < 2^53)
+// acc += (-1)^neg (m1 m2 >> r) mod 2^64, r >= 0 (m1, m2 < 2^53). The factors'
+// high words have 21 bits, so the middle products add without a carry and the
+// 106-bit product takes four 32 x 32-bit multiplies and two additions; the shift
+// picks three of its words by r's two high bits and funnels them by the rest.
 __device__ __forceinline__ void mod_mac(unsigned long long &acc, unsigned long long m1,
                                         unsigned long long m2, int r, bool neg) {
-  const unsigned long long lo = m1 * m2, hi = __umul64hi(m1, m2);
+  const unsigned l1 = (unsigned)m1, h1 = (unsigned)(m1 >> 32);
+  const unsigned l2 = (unsigned)m2, h2 = (unsigned)(m2 >> 32);
+  const unsigned long long p0 = (unsigned long long)l1 * l2;
+  const unsigned long long p1 =
+      (unsigned long long)h1 * l2 + (unsigned long long)l1 * h2 + (p0 >> 32);
+  const unsigned long long p2 = (unsigned long long)h1 * h2 + (p1 >> 32);
+  const unsigned w0 = (unsigned)p0, w1 = (unsigned)p1, w2 = (unsigned)p2,
+                 w3 = (unsigned)(p2 >> 32);
   const int rr = min(r, 127);
-  const unsigned long long v =
-      rr >= 64 ? (hi >> (rr - 64)) : ((lo >> rr) | ((hi << 1) << (63 - rr)));
+  const bool q1 = (rr & 64) != 0, q0 = (rr & 32) != 0;
+  const unsigned x0 = q1 ? w2 : w0, x1 = q1 ? w3 : w1, x2 = q1 ? 0u : w2, x3 = q1 ? 0u : w3;
+  const unsigned y0 = q0 ? x1 : x0, y1 = q0 ? x2 : x1, y2 = q0 ? x3 : x2;
+  const unsigned v0 = __funnelshift_r(y0, y1, rr), v1 = __funnelshift_r(y1, y2, rr);
+  const unsigned long long v = ((unsigned long long)v1 << 32) | v0;
   acc = neg ? acc - v : acc + v;
 }
 // acc += (-1)^neg (m << s) mod 2^64 (s < 64; s < 0 shifts right)

@@ -492,8 +492,10 @@ __global__ void __launch_bounds__(tile_max_warps(N) * 32, tile_min_ctas(N))
 // critical path.
 // COPY: the entries carry the matrix (the host-link variant's list), which is
 // the source of the residual instead of src.
+// Compiled for 8 CTAs per SM (32768 LLL x n=24, us: 114 without a bound, 107.5
+// for 8, 111 for 9; n = 32 the same, whose shared memory allows 8).
 template <int N, class Src, bool COPY = false>
-__global__ void __launch_bounds__(kFacCorrectWarps * 32)
+__global__ void __launch_bounds__(kFacCorrectWarps * 32, 8)
     lup_mixed_fac_correct_kernel(Src src, const CallHead *head, const unsigned char *fac,
                                  long long fac_cap, double *__restrict__ logabs,
                                  double *__restrict__ phase, int8_t *__restrict__ parity,

@@ -77,7 +77,7 @@ constexpr int kPlanDeferMinN = 24;
 
 // A plan's passes (see Launch), and the largest n of a mixed plan's small
 // pass (grouped_small_kernel: the lane-grid path, several matrices per warp).
-constexpr int kPlanPasses = 6;
+constexpr int kPlanPasses = 4;
 constexpr int kSmallPassMaxN = 16;
 
 struct WorkItem {
@@ -94,8 +94,8 @@ struct WorkItem {
 // Shared memory of one warp, contiguous: [matrix area][F][hold][er, ec].
 //  * matrix area: the FP64 matrix (double2, nf x (nf+1)) for the FP64 routine,
 //    aliased by the FP32 path's hi/lo copy (float4, nm x (nm+1));
-//  * F: the FP32 factor (float2, at most nm x (nm+2)); hold: 2 nf doubles;
-//    er, ec: 2 nm ints.
+//  * F: the FP32 factor (float2, nm x (nm+1)); hold: 2 nf doubles; er, ec:
+//    2 nm ints.
 // nf is the largest n of the plan, nm the largest n that takes the FP32 path
 // (0 in the plain modes and for groups the precision policy sends to FP64),
 // so a group that only runs the FP64 routine costs the plain kernel's bytes.
@@ -108,7 +108,7 @@ __host__ __device__ inline WarpLayout warp_layout(int nm, int nf) {
   const size_t a_fp64 = (size_t)nf * (nf + 1) * sizeof(double2);
   const size_t a_fp32 = (size_t)nm * (nm + 1) * sizeof(float4);
   L.area = a_fp64 > a_fp32 ? a_fp64 : a_fp32;
-  L.f = (size_t)nm * (nm + 2) * sizeof(float2);
+  L.f = (size_t)nm * (nm + 1) * sizeof(float2);
   L.hold = 2 * (size_t)nf * sizeof(double);
   const size_t ints = 2 * (size_t)nm * sizeof(int);
   L.total = (L.area + L.f + L.hold + ints + 15) & ~(size_t)15;
@@ -158,12 +158,25 @@ __device__ void process_matrix(const double2 *src, int n, int lda, long long ob,
     return;
   }
   if (MODE == LUFQHE_MODE_MIXED) {
-    // (n <= kSmallPassMaxN, 24 and 32 have passes of their own)
     CFF prod;
     int exp_sum = 0, par = 0;
     float2 corr;
-    const MixedSmem S{F, HL, hold, er, ec};
-    if (mixed_factor(S, n, lane, theta2, prod, exp_sum, corr, par))
+    bool ok;
+    switch (n) {
+      // (n <= kSmallPassMaxN goes to the small pass)
+      case 24: ok = mixed_factor_tile<24>(HL, F, er, ec, lane, theta2, prod, exp_sum, corr, par, refine); break;
+      case 32: ok = mixed_factor_tile<32>(HL, F, er, ec, lane, theta2, prod, exp_sum, corr, par, refine); break;
+      default: {
+        MixedSmem S;
+        S.SC = HL;
+        S.Af = F;
+        S.hold = hold;
+        S.er = er;
+        S.ec = ec;
+        ok = mixed_factor(S, n, lane, theta2, prod, exp_sum, corr, par);
+      }
+    }
+    if (ok)
       out.push(lane, ob, prod, exp_sum, corr, par, logabs, phase, parity, status);
     else
       plan_fp64(src, n, lda, ob, M, hold, lane, LUFQHE_ST_FALLBACK, cs, fl, aux, logabs, phase,
@@ -305,85 +318,15 @@ __global__ void __launch_bounds__(kMaxWarpsMixed * 32, 2)
   out.flush(lane, logabs, phase, parity, status);
 }
 
-// A mixed plan's pass over its groups of n = 24 or of n = 32 on the FP32 path, in
-// that size's own shared memory and registers, on the lane grid as the batched
-// mixed mode (one pass for both had n = 24 at the 8 warps per SM that n = 32's
-// shared memory allows, where 15 fit: 979 us for 7000 LLL matrices of each, now
-// 286 and 657, and their pending pass 281 -> 225); a matrix to refine is refined
-// here.
-constexpr int tile_pass_warps(int n) { return n == 24 ? 3 : 4; }
-template <int N>
-__global__ void __launch_bounds__(tile_pass_warps(N) * 32, N == 24 ? 5 : 3)
-    grouped_tile_kernel(const WorkItem *__restrict__ items, int nitems, unsigned int *counter,
-                        int nm, int nf, float theta2, int refine, double *__restrict__ logabs,
-                        double *__restrict__ phase, int8_t *__restrict__ parity,
-                        int32_t *__restrict__ status, PlanAux aux) {
-  (void)nm;
-  (void)nf;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const WarpLayout L = warp_layout(N, N);
-  unsigned char *base = smem_raw + (size_t)warp * L.total;
-  float4 *HL = reinterpret_cast<float4 *>(base);
-  double2 *M = reinterpret_cast<double2 *>(HL);
-  float2 *F = reinterpret_cast<float2 *>(base + L.area);
-  double *hold = reinterpret_cast<double *>(base + L.area + L.f);
-  int *ints = reinterpret_cast<int *>(base + L.area + L.f + L.hold);
-  const CorrScratch cs{F, ints, hold};
-  const FacList *fl = aux.lists && aux.lists[N].count ? aux.lists + N : nullptr;
-
-  DeferredOut out;
-  for (;;) {
-    unsigned int it = 0;
-    if (lane == 0) it = atomicAdd(counter, 1u);
-    it = __shfl_sync(kFull, it, 0);
-    if (it >= (unsigned int)nitems) break;
-    const WorkItem w = items[it];
-    for (int j = 0; j < w.count; ++j) {
-      const double2 *src = w.A + (size_t)(w.first + j) * N * w.lda;
-      const long long ob = w.out + j;
-      __syncwarp();
-      if (route_fp64(src, w.share64k)) {
-        plan_fp64(src, N, w.lda, ob, M, hold, lane, LUFQHE_ST_FP64, cs, fl, aux, logabs, phase,
-                  parity, status);
-        continue;
-      }
-      load_rows(DenseSource{src, w.lda}, 0, N, N, M, N + 1, N, lane);
-      __syncwarp();
-      grid_unit<N, 32, N, false, false>(
-          DenseSource{src, w.lda}, 0, ob, 1, N, HL, F, ints, lane, theta2, 0u, refine != 0,
-          [&](long long, bool, bool can_refine, const CFF &prod, int exp_sum, int par) {
-            if (can_refine) {
-              float2 *Rm = reinterpret_cast<float2 *>(HL);
-              float2 corr;
-              repack_f<N, N>(F, lane);
-              if (mixed_refine_tile<N>(F, Rm, Rm + N * (N + 1), reinterpret_cast<float2 *>(ints),
-                                       lane, theta2, tile_la_est(prod, exp_sum), corr)) {
-                out.push(lane, ob, prod, exp_sum, corr, par, logabs, phase, parity, status);
-                return;
-              }
-            }
-            plan_fp64(src, N, w.lda, ob, M, hold, lane, LUFQHE_ST_FALLBACK, cs, fl, aux, logabs,
-                      phase, parity, status);
-          },
-          out, logabs, phase, parity, status);
-    }
-  }
-  out.flush(lane, logabs, phase, parity, status);
-}
-
 using GroupedKernel = void (*)(const WorkItem *, int, unsigned int *, int, int, float, int,
                                double *, double *, int8_t *, int32_t *, PlanAux);
 
-GroupedKernel kernel_for(int mode, int pass = 0) {
-  if (pass == 3) return grouped_small_kernel;
-  if (pass == 4) return grouped_tile_kernel<24>;
-  if (pass == 5) return grouped_tile_kernel<32>;
+GroupedKernel kernel_for(int mode, bool small = false) {
   switch (mode) {
     case LUFQHE_MODE_PLAIN_FP64: return grouped_kernel<LUFQHE_MODE_PLAIN_FP64>;
     case LUFQHE_MODE_PLAIN_FP64_FUSED: return grouped_kernel<LUFQHE_MODE_PLAIN_FP64_FUSED>;
     default:
-      return grouped_kernel<LUFQHE_MODE_MIXED>;
+      return small ? grouped_small_kernel : grouped_kernel<LUFQHE_MODE_MIXED>;
   }
 }
 
@@ -518,8 +461,8 @@ GroupedKernel group_kernel_for(int mode, bool correct) {
                                         : grouped_group_kernel<ARITH_FUSED>;
 }
 
-// One pass of a plan: a grouped kernel over its own work list. A plan runs these
-// passes back to back:
+// One pass of a plan: a grouped kernel over its own work list. A plan runs up
+// to three passes back to back:
 //  0. the plan's mode over the groups on the warp-per-matrix path (a mixed
 //     plan's FP32-path groups; a plain plan's groups with n <= 32);
 //  1. (mixed plans) the plain fused kernel over the groups with n <= 32 that
@@ -527,8 +470,7 @@ GroupedKernel group_kernel_for(int mode, bool correct) {
 //  2. the warp-group kernel over the FP64-route groups with n > 32 (fused
 //     arithmetic for a mixed plan, the plan's arithmetic for a plain one);
 //  3. (mixed plans) grouped_small_kernel over the FP32-path groups with
-//     n <= kSmallPassMaxN;
-//  4, 5. (mixed plans) grouped_tile_kernel over those of n = 24 and of n = 32.
+//     n <= kSmallPassMaxN.
 // Groups routed to FP64 need neither the FP32 path's shared memory nor its
 // registers, and get the plain kernels' occupancy. After the passes a mixed
 // plan runs its pending pass (grouped_pending_kernel) and the correction
@@ -600,9 +542,7 @@ int pass_of(const lufqhe_plan_s *p, size_t g) {
   const bool fp64 = p->mode != LUFQHE_MODE_MIXED || p->share[g] >= 65536u;
   if (fp64 && p->groups[g].n >= kFp64GroupMinN) return 2;
   if (p->mode == LUFQHE_MODE_MIXED && fp64) return 1;
-  if (p->mode != LUFQHE_MODE_MIXED) return 0;
-  const int n = p->groups[g].n;
-  return n <= kSmallPassMaxN ? 3 : n == 24 ? 4 : n == 32 ? 5 : 0;
+  return p->mode == LUFQHE_MODE_MIXED && p->groups[g].n <= kSmallPassMaxN ? 3 : 0;
 }
 
 int build_items(lufqhe_plan_s *p, cudaStream_t s) {
@@ -623,7 +563,7 @@ int build_items(lufqhe_plan_s *p, cudaStream_t s) {
       w.count = (int)std::min<long long>(T, G.count - f);
       w.n = G.n;
       w.lda = G.lda;
-      const bool fp32_path = pass == 0 || pass >= 3;
+      const bool fp32_path = pass == 0 || pass == 3;
       w.share64k = p->mode == LUFQHE_MODE_MIXED && fp32_path ? p->share[g] : 0u;
       w.status_or = p->mode == LUFQHE_MODE_MIXED && !fp32_path ? LUFQHE_ST_FP64 : 0;
       items[pass].push_back(w);
@@ -705,9 +645,8 @@ int configure_pass(lufqhe_plan_s *p, int pass, int warps) {
     L.ctas = device_sm_count() * per_sm;
     return LUFQHE_SUCCESS;
   }
-  GroupedKernel k = kernel_for(L.mode, pass);
+  GroupedKernel k = kernel_for(L.mode, pass == 3);
   const size_t per_warp = pass == 3 ? small_warp_bytes(L.nm) : warp_layout(L.nm, L.nf).total;
-  if (pass > 3) warps = tile_pass_warps(L.nf);
   const size_t optin = device_smem_optin();
   int w = std::min<int>(warps, (int)(optin / per_warp));
   if (w < 1) {
@@ -753,13 +692,12 @@ int launch_once(lufqhe_plan_s *p, cudaStream_t s) {
     const Launch &L = p->launch[pass];
     if (L.nitems == 0 || L.ctas == 0) continue;
     GroupedKernel k =
-        pass == 2 ? group_kernel_for(L.mode, L.nm > 0) : kernel_for(L.mode, pass);
+        pass == 2 ? group_kernel_for(L.mode, L.nm > 0) : kernel_for(L.mode, pass == 3);
     // a warp-group CTA takes one item at a time
     const long long want = pass == 2 ? L.nitems : (L.nitems + L.warps - 1) / L.warps;
     const int grid = (int)std::min<long long>(L.ctas, want);
     static const char *names[kPlanPasses] = {"grouped_kernel", "grouped_kernel_fp64",
-                                             "grouped_group_kernel", "grouped_kernel_small",
-                                             "grouped_tile_kernel", "grouped_tile_kernel"};
+                                             "grouped_group_kernel", "grouped_kernel_small"};
     KernelTimer timer(names[pass], L.nf, s);
     k<<<std::max(1, grid), L.warps * 32, L.smem, s>>>(p->d_items + L.first, L.nitems,
                                                        p->d_counter + pass, L.nm, L.nf, p->theta2,

@@ -70,17 +70,6 @@ struct GridLane {
   __device__ __forceinline__ int at(int rr, int cc) const { return gb + rr * Grid<NP, LPM>::GC + cc; }
 };
 
-// cfms and cmulf as packed pairs: the same rounded operations in half the
-// instructions (broadcast, exchanged and negated operands cost nothing extra).
-__device__ __forceinline__ float2 cfms2(float2 s, float2 l, float2 u) {
-  s = f2fma(make_float2(-l.x, -l.x), u, s);
-  return f2fma(make_float2(l.y, -l.y), make_float2(u.y, u.x), s);
-}
-__device__ __forceinline__ float2 cmulf2(float2 a, float2 b) {
-  const float2 t = f2mul(make_float2(-a.y, a.y), make_float2(b.y, b.x));
-  return f2fma(make_float2(a.x, a.x), b, t);
-}
-
 template <int LPM>
 __device__ __forceinline__ unsigned group_max(unsigned v) {
   if constexpr (LPM == 32) {

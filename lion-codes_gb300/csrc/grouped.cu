@@ -75,10 +75,8 @@ struct PlanAux {
 // (as the batched mixed mode leaves them to its finish kernel from n = 24).
 constexpr int kPlanDeferMinN = 24;
 
-// A plan's passes (see Launch), and the largest n of a mixed plan's small
-// pass (grouped_small_kernel: the lane-grid path, several matrices per warp).
+// A plan's passes (see Launch).
 constexpr int kPlanPasses = 4;
-constexpr int kSmallPassMaxN = 16;
 
 struct WorkItem {
   const double2 *A;  // group base
@@ -173,7 +171,7 @@ __device__ void process_matrix(const double2 *src, int n, int lda, long long ob,
     float2 corr;
     bool ok;
     switch (n) {
-      // (n <= kSmallPassMaxN goes to the small pass)
+      // (n <= kSmallMaxN goes to the small pass)
       case 24: ok = tile_call<24>(HL, F, er, ec, lane, theta2, &prod, &exp_sum, &corr, &par, refine); break;
       case 32: ok = tile_call<32>(HL, F, er, ec, lane, theta2, &prod, &exp_sum, &corr, &par, refine); break;
       default: {
@@ -263,22 +261,15 @@ __global__ void __launch_bounds__(kMaxWarpsMixed * 32, 1)
   out.flush(lane, logabs, phase, parity, status);
 }
 
-// A mixed plan's small pass: the FP32-path groups with n <= kSmallPassMaxN, each
+// A mixed plan's small pass: the FP32-path groups with n <= kSmallMaxN, each
 // warp taking an item's matrices several at a time (the batched call's path and
-// bits). nm sizes a warp's shared memory.
-__host__ __device__ constexpr size_t small_warp_bytes(int nm) {
-  return nm <= 8 ? Grid<8, 8>::kWarpBytes
-         : nm <= 12 ? (Grid<12, 16>::kWarpBytes > Grid<8, 8>::kWarpBytes
-                           ? Grid<12, 16>::kWarpBytes
-                           : Grid<8, 8>::kWarpBytes)
-                    : Grid<16, 16>::kWarpBytes;
-}
-
-template <int NP, int LPM, int NC>
+// bits, on its grid of the size). nm, the pass's largest n, sizes a warp's
+// shared memory.
+template <int NP, int NC>
 __device__ void small_item(const WorkItem &w, unsigned char *base, int lane, float theta2,
                            bool refine, DeferredOut &out, double *logabs, double *phase,
                            int8_t *parity, int32_t *status) {
-  using Gd = Grid<NP, LPM>;
+  using Gd = SmallGrid<NP>;
   float4 *HLw = reinterpret_cast<float4 *>(base);
   float2 *Fw = reinterpret_cast<float2 *>(HLw + Gd::G * Gd::kHL);
   int *Iw = reinterpret_cast<int *>(Fw + Gd::G * Gd::kF);
@@ -289,9 +280,9 @@ __device__ void small_item(const WorkItem &w, unsigned char *base, int lane, flo
     __syncwarp();
     load_rows(src, w.first + j, cnt * n, n, reinterpret_cast<double2 *>(HLw), Gd::LDH, NP, lane);
     __syncwarp();
-    grid_unit<NP, LPM, NC, true, true>(src, w.first + j, w.out + j, cnt, n, HLw, Fw, Iw, lane, theta2,
-                                 w.share64k, refine, [](long long, bool, bool, const CFF &, int, int) {}, out, logabs, phase,
-                                 parity, status);
+    grid_unit<NP, Gd::LPM, NC, true, true>(
+        src, w.first + j, w.out + j, cnt, n, HLw, Fw, Iw, lane, theta2, w.share64k, refine,
+        [](long long, bool, bool, const CFF &, int, int) {}, out, logabs, phase, parity, status);
   }
 }
 
@@ -314,15 +305,16 @@ __global__ void __launch_bounds__(kMaxWarpsMixed * 32, 2)
     const WorkItem w = items[it];
     const bool rf = refine != 0;
     switch (w.n) {
-      case 6: small_item<8, 8, 6>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
-      case 8: small_item<8, 8, 8>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
-      case 12: small_item<12, 16, 12>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
-      case 16: small_item<16, 16, 16>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
+      case 6: small_item<8, 6>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
+      case 8: small_item<8, 8>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
+      case 12: small_item<12, 12>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
+      case 16: small_item<16, 16>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
       default:
-        if (w.n < 8)
-          small_item<8, 8, 0>(w, base, lane, theta2, rf, out, logabs, phase, parity, status);
-        else
-          small_item<16, 16, 0>(w, base, lane, theta2, rf, out, logabs, phase, parity, status);
+        switch (small_np(w.n)) {
+          case 8: small_item<8, 0>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
+          case 12: small_item<12, 0>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
+          default: small_item<16, 0>(w, base, lane, theta2, rf, out, logabs, phase, parity, status);
+        }
     }
   }
   out.flush(lane, logabs, phase, parity, status);
@@ -345,7 +337,7 @@ GroupedKernel kernel_for(int mode, bool small = false) {
 // unit, and a group of 7000 matrices of n = 6 in items of 152 had kept 46 of
 // 2432 warps busy).
 int default_tile(int n, int mode) {
-  if (mode == LUFQHE_MODE_MIXED && n <= kSmallPassMaxN) return n <= 8 ? 8 : 4;
+  if (mode == LUFQHE_MODE_MIXED && n <= kSmallMaxN) return n <= 8 ? 8 : 4;
   double t = 64.0 * std::pow(8.0 / (double)n, 3.0);
   int v = (int)std::lround(t);
   return std::max(1, std::min(256, v));
@@ -480,7 +472,7 @@ GroupedKernel group_kernel_for(int mode, bool correct) {
 //  2. the warp-group kernel over the FP64-route groups with n > 32 (fused
 //     arithmetic for a mixed plan, the plan's arithmetic for a plain one);
 //  3. (mixed plans) grouped_small_kernel over the FP32-path groups with
-//     n <= kSmallPassMaxN.
+//     n <= kSmallMaxN.
 // Groups routed to FP64 need neither the FP32 path's shared memory nor its
 // registers, and get the plain kernels' occupancy. After the passes a mixed
 // plan runs its pending pass (grouped_pending_kernel) and the correction
@@ -552,7 +544,7 @@ int pass_of(const lufqhe_plan_s *p, size_t g) {
   const bool fp64 = p->mode != LUFQHE_MODE_MIXED || p->share[g] >= 65536u;
   if (fp64 && p->groups[g].n >= kFp64GroupMinN) return 2;
   if (p->mode == LUFQHE_MODE_MIXED && fp64) return 1;
-  return p->mode == LUFQHE_MODE_MIXED && p->groups[g].n <= kSmallPassMaxN ? 3 : 0;
+  return p->mode == LUFQHE_MODE_MIXED && p->groups[g].n <= kSmallMaxN ? 3 : 0;
 }
 
 int build_items(lufqhe_plan_s *p, cudaStream_t s) {

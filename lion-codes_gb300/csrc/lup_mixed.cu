@@ -44,7 +44,7 @@ int g_mixed_refine = 1;
 size_t mixed_workspace_bytes(int n, long long batch) {
   if (fp64_share_64k(n) >= 65536u || batch == 0) return 0;
   auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
-  if (n <= 16) return kHeadBytes;  // at most the work counter
+  if (n <= kSmallMaxN) return kHeadBytes;  // at most the work counter
   size_t bytes = kHeadBytes + up((size_t)batch * sizeof(unsigned int));
   if (g_mixed_refine && (n == 24 || n == 32)) {
     long long cap = std::max<long long>(256, (long long)(kRefineShare * (double)batch));

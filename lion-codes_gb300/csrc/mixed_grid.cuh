@@ -53,6 +53,35 @@ struct Grid {
       G * (kHL * sizeof(float4) + kF * sizeof(float2) + 2 * NP * sizeof(int));
 };
 
+// The grid of a size n <= 16: padded to NP = 8, 12 or 16, whichever path takes
+// it. The kernels dispatch by small_np and reserve small_warp_bytes; both follow
+// from here.
+constexpr int kSmallMaxN = 16;
+__host__ __device__ constexpr int small_np(int n) { return n <= 8 ? 8 : n <= 12 ? 12 : 16; }
+template <int NP>
+using SmallGrid = Grid<NP, NP == 8 ? 8 : 16>;
+// Shared memory of a warp on size n's grid, and of one that takes every size up
+// to nm.
+__host__ __device__ constexpr size_t small_layout_bytes(int n) {
+  return small_np(n) == 8    ? SmallGrid<8>::kWarpBytes
+         : small_np(n) == 12 ? SmallGrid<12>::kWarpBytes
+                             : SmallGrid<16>::kWarpBytes;
+}
+__host__ __device__ constexpr size_t small_warp_bytes(int nm) {
+  size_t most = 0;
+  for (int n = 1; n <= nm; ++n)
+    if (small_layout_bytes(n) > most) most = small_layout_bytes(n);
+  return most;
+}
+// Every size fits its grid, and the reservation covers it for every nm >= n.
+constexpr bool small_layouts_covered() {
+  for (int nm = 1; nm <= kSmallMaxN; ++nm)
+    for (int n = 1; n <= nm; ++n)
+      if (small_np(n) < n || small_warp_bytes(nm) < small_layout_bytes(n)) return false;
+  return true;
+}
+static_assert(small_layouts_covered(), "a warp's shared memory must hold every size it takes");
+
 // This lane's place in its matrix's grid.
 template <int NP, int LPM>
 struct GridLane {

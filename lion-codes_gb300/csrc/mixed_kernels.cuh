@@ -837,9 +837,10 @@ int launch_mixed_grid(Src src, int n, long long batch, float theta2, double *log
 // n <= 16: several matrices per warp, except in a batch of at most one matrix
 // per SM sub-partition, where a warp each has the least latency (64 LLL matrices
 // of n = 16: 23.2 us a call with two per warp, 18.7 us with one).
-template <int NP, int LPM, int NC, class Src>
+template <int NP, int NC, class Src>
 int launch_mixed_small(Src src, int n, long long batch, float theta2, double *logabs,
                        double *phase, int8_t *parity, int32_t *status, cudaStream_t stream) {
+  constexpr int LPM = SmallGrid<NP>::LPM;
   constexpr int NP1 = NP == 12 ? 16 : NP;  // whole 8-column slots
   if (batch <= 4ll * device_sm_count())
     return launch_mixed_grid<NP1, 32, NC, false>(src, n, batch, theta2, logabs, phase, parity,
@@ -868,10 +869,10 @@ int launch_mixed_src(Src src, int n, long long batch, double *logabs, double *ph
   const float th2 = g_mixed_theta * g_mixed_theta;
   if constexpr (has_even_n<Src>::value) {
     switch (n) {
-      case 6: return launch_mixed_small<8, 8, 6>(src, n, batch, th2, logabs, phase, parity, status, stream);
-      case 8: return launch_mixed_small<8, 8, 8>(src, n, batch, th2, logabs, phase, parity, status, stream);
-      case 12: return launch_mixed_small<12, 16, 12>(src, n, batch, th2, logabs, phase, parity, status, stream);
-      case 16: return launch_mixed_small<16, 16, 16>(src, n, batch, th2, logabs, phase, parity, status, stream);
+      case 6: return launch_mixed_small<8, 6>(src, n, batch, th2, logabs, phase, parity, status, stream);
+      case 8: return launch_mixed_small<8, 8>(src, n, batch, th2, logabs, phase, parity, status, stream);
+      case 12: return launch_mixed_small<12, 12>(src, n, batch, th2, logabs, phase, parity, status, stream);
+      case 16: return launch_mixed_small<16, 16>(src, n, batch, th2, logabs, phase, parity, status, stream);
       case 24:
         if constexpr (std::is_same<Src, DenseSource>::value)
           if (inplace) return launch_mixed_hostlink<24>(src, batch, th2, logabs, phase, parity, status, stream);
@@ -884,9 +885,13 @@ int launch_mixed_src(Src src, int n, long long batch, double *logabs, double *ph
     }
   }
   // other sizes on the lane grid of the next size up
-  if (n <= 8) return launch_mixed_small<8, 8, 0>(src, n, batch, th2, logabs, phase, parity, status, stream);
-  if (n <= 12) return launch_mixed_small<12, 16, 0>(src, n, batch, th2, logabs, phase, parity, status, stream);
-  if (n <= 16) return launch_mixed_small<16, 16, 0>(src, n, batch, th2, logabs, phase, parity, status, stream);
+  if (n <= kSmallMaxN) {
+    switch (small_np(n)) {
+      case 8: return launch_mixed_small<8, 0>(src, n, batch, th2, logabs, phase, parity, status, stream);
+      case 12: return launch_mixed_small<12, 0>(src, n, batch, th2, logabs, phase, parity, status, stream);
+      default: return launch_mixed_small<16, 0>(src, n, batch, th2, logabs, phase, parity, status, stream);
+    }
+  }
   if (n <= 24) return launch_mixed_grid<24, 32, 0, true>(src, n, batch, th2, logabs, phase, parity, status, stream);
   if (n <= 32) return launch_mixed_grid<32, 32, 0, true>(src, n, batch, th2, logabs, phase, parity, status, stream);
   const size_t per_warp = mixed_smem_per_warp(n);

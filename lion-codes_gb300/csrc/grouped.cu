@@ -275,13 +275,36 @@ __device__ void small_item(const WorkItem &w, unsigned char *base, int lane, flo
   int *Iw = reinterpret_cast<int *>(Fw + Gd::G * Gd::kF);
   const DenseSource src{w.A, w.lda};
   const int n = NC ? NC : w.n;
-  for (int j = 0; j < w.count; j += Gd::G) {
-    const int cnt = min(Gd::G, w.count - j);
+  double2 *M = reinterpret_cast<double2 *>(HLw);
+  for (int j = 0; j < w.count;) {
+    // the unit: G consecutive matrices, or, where a share is routed to FP64, the
+    // next G that are not (the ones in between go to FP64 on the way)
+    int cnt = 0, mine = 0;
+    if (!w.share64k) {
+      cnt = min(Gd::G, w.count - j);
+      mine = j + lane / Gd::LPM;
+      j += cnt;
+    }
+    for (; w.share64k && cnt < Gd::G && j < w.count; ++j) {
+      if (route_fp64_entry(src.first(w.first + j, n), w.share64k)) {
+        grid_refactor_call<NP>(src, w.first + j, n, HLw, Fw, lane, w.out + j, logabs, phase,
+                               parity, status, LUFQHE_ST_FP64);
+      } else {
+        if (cnt == lane / Gd::LPM) mine = j;
+        ++cnt;
+      }
+    }
+    if (cnt == 0) break;
+    auto at = [&](int q) { return __shfl_sync(kFull, mine, q * Gd::LPM); };
     __syncwarp();
-    load_rows(src, w.first + j, cnt * n, n, reinterpret_cast<double2 *>(HLw), Gd::LDH, NP, lane);
+    if (!w.share64k)
+      load_rows(src, w.first + at(0), cnt * n, n, M, Gd::LDH, NP, lane);
+    else
+      for (int q = 0; q < cnt; ++q)
+        load_rows(src, w.first + at(q), n, n, M + q * Gd::kHL, Gd::LDH, NP, lane);
     __syncwarp();
     grid_unit<NP, Gd::LPM, NC, true, true>(
-        src, w.first + j, w.out + j, cnt, n, HLw, Fw, Iw, lane, theta2, w.share64k, refine,
+        src, w.first, w.out, cnt, n, HLw, Fw, Iw, lane, theta2, 0u, refine, at,
         [](long long, bool, bool, const CFF &, int, int) {}, out, logabs, phase, parity, status);
   }
 }

@@ -1,5 +1,5 @@
-// Mixed-precision batched complex LUP determinant: complex128 and
-// lowest-Landau-level entry points, the precision policy and the options.
+// Mixed-precision batched complex LUP determinant: the complex128 entry point,
+// the precision policy and the options.
 // The method and its kernels are described in mixed_kernels.cuh.
 
 #include <cstddef>
@@ -39,12 +39,12 @@ float g_mixed_theta = 0.1f;
 int g_mixed_refine = 1;
 
 // Device memory a batched mixed call takes from the library's pool while it
-// runs, its state block (CallState): the head, for n >= 17 the pending list
-// (one entry per matrix) and, for n = 24 and 32, the saved matrices.
+// runs, its state block (CallState): the head, for n >= 17 or a routed share the
+// pending list (one entry per matrix) and, for n = 24 and 32, the saved matrices.
 size_t mixed_workspace_bytes(int n, long long batch) {
   if (fp64_share_64k(n) >= 65536u || batch == 0) return 0;
   auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
-  if (n <= kSmallMaxN) return kHeadBytes;  // at most the work counter
+  if (n <= kSmallMaxN && !fp64_share_64k(n)) return kHeadBytes;  // at most the work counter
   size_t bytes = kHeadBytes + up((size_t)batch * sizeof(unsigned int));
   if (g_mixed_refine && (n == 24 || n == 32)) {
     long long cap = std::max<long long>(256, (long long)(kRefineShare * (double)batch));
@@ -89,13 +89,5 @@ int launch_listed_corrections(int n, const void *head, const unsigned char *list
 }
 size_t listed_count_offset() { return offsetof(CallHead, corr_count); }
 size_t head_bytes() { return kHeadBytes; }
-
-int launch_mixed_lll(const double2 *Z, int n, long long batch, double *logabs, double *phase,
-                     int8_t *parity, int32_t *status, cudaStream_t stream) {
-  return launch_mixed_src(LllSource{Z}, n, batch, logabs, phase, parity, status, stream, [&] {
-    return launch_plain_lll(Z, n, batch, ARITH_FUSED, logabs, phase, parity, status, stream,
-                            LUFQHE_ST_FP64);
-  });
-}
 
 }  // namespace lufqhe

@@ -607,7 +607,11 @@ __device__ void fallback_fp64_src(const Src &src, long long sb, int n, double2 *
                                   const CorrScratch *cs = nullptr,
                                   const FacList *fl = nullptr) {
   __syncwarp();
-  src.template load<COHERENT>(sb, n, M, lds, lane);
+  // (a matrix routed here was not looked at before)
+  if (src.template load<COHERENT>(sb, n, M, lds, lane)) {
+    emit_nonfinite(lane, b, logabs, phase, parity, status);
+    return;
+  }
   int par = 0;
   const bool correct = cs != nullptr && n >= kCorrectMinN && n <= kCorrectMaxN;
   int st = lup_fp64_warp<ARITH_FUSED>(M, lds, hold, n, lane, &par, correct ? cs->ints : nullptr);

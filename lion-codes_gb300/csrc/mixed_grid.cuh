@@ -771,15 +771,17 @@ __device__ __noinline__ void grid_refactor_call(const Src src, long long sb, int
   grid_refactor<NP>(src, sb, n, HL, F, lane, ob, logabs, phase, parity, status, flag);
 }
 
-// The `cnt` matrices from b0 of src, staged in the warp's area (group q at
-// HLw + q kHL), into outputs ob0 ..: the FP32 path, then what it does not accept:
-// refined or refactorised right here (INPLACE, n <= 16), or handed to
-// defer(b, routed, can_refine, prod, exp_sum, par). share64k: the share routed
-// straight to FP64. CALL: FP64 out of line.
-template <int NP, int LPM, int NC, bool INPLACE, bool CALL, class Src, class Defer>
+// One unit of a warp: matrices b0 + at(q), q < cnt, of src, staged in areas
+// HLw + q kHL, into outputs ob0 + at(q): the FP32 path, then what it does not
+// accept: refined or refactorised right here (INPLACE, n <= 16), or handed to
+// defer(b, routed, can_refine, prod, exp_sum, par). share64k: the share routed to
+// FP64, of which several matrices per warp may hold a part: they go to defer in
+// any case (the kernels ask for units of such matrices alone before they stage
+// them). CALL: FP64 out of line.
+template <int NP, int LPM, int NC, bool INPLACE, bool CALL, class Src, class At, class Defer>
 __device__ __forceinline__ void grid_unit(const Src &src, long long b0, long long ob0, int cnt,
                                           int n, float4 *HLw, float2 *Fw, int *Iw, int lane,
-                                          float theta2, unsigned int share64k, bool refine,
+                                          float theta2, unsigned int share64k, bool refine, At at,
                                           Defer defer, DeferredOut &out, double *logabs,
                                           double *phase, int8_t *parity, int32_t *status) {
   using Gd = Grid<NP, LPM>;
@@ -787,11 +789,10 @@ __device__ __forceinline__ void grid_unit(const Src &src, long long b0, long lon
   CFF prod;
   int exp_sum, par;
   float2 corr;
-  int code = grid_factor<NP, LPM, NC>(HLw + grp * Gd::kHL, Fw + grp * Gd::kF,
-                                               Iw + grp * 2 * NP, n, lane, theta2, prod, exp_sum,
-                                               corr, par);
+  int code = grid_factor<NP, LPM, NC>(HLw + grp * Gd::kHL, Fw + grp * Gd::kF, Iw + grp * 2 * NP, n,
+                                      lane, theta2, prod, exp_sum, corr, par);
   bool routed = false;
-  if (share64k && grp < cnt && code != TILE_NONFINITE) {
+  if (Gd::G > 1 && share64k && grp < cnt && code != TILE_NONFINITE) {
     routed = route_fp64_entry(src.first(b0 + grp, n), share64k);
     if (routed) code = TILE_REJECT;
   }
@@ -808,7 +809,7 @@ __device__ __forceinline__ void grid_unit(const Src &src, long long b0, long lon
       rq = __shfl_sync(kFull, par, from);
       kq = shfl2(corr, from);
     }
-    const long long ob = ob0 + q;
+    const long long b = b0 + at(q), ob = ob0 + at(q);
     if (cq == TILE_ACCEPT) {
       out.push(lane, ob, pq, eq, kq, rq, logabs, phase, parity, status);
       continue;
@@ -817,9 +818,11 @@ __device__ __forceinline__ void grid_unit(const Src &src, long long b0, long lon
       emit_nonfinite(lane, ob, logabs, phase, parity, status);
       continue;
     }
-    const bool rt = Gd::G > 1 ? __shfl_sync(kFull, (int)routed, from) != 0 : routed;
+    const bool rt = Gd::G > 1 && share64k && __shfl_sync(kFull, (int)routed, from) != 0;
     if constexpr (!INPLACE) {
-      defer(b0 + q, rt, cq == TILE_REFINE && refine, pq, eq, rq);
+      defer(b, rt, cq == TILE_REFINE && refine, pq, eq, rq);
+    } else if (rt) {
+      defer(b, true, false, pq, eq, rq);
     } else {
       float4 *HLq = HLw + q * Gd::kHL;
       float2 *Fq = Fw + q * Gd::kF;
@@ -835,12 +838,12 @@ __device__ __forceinline__ void grid_unit(const Src &src, long long b0, long lon
           }
         }
       }
-      const int flag = rt ? LUFQHE_ST_FP64 : LUFQHE_ST_FALLBACK;
       if constexpr (CALL)
-        grid_refactor_call<NP>(src, b0 + q, n, HLq, Fq, lane, ob, logabs, phase, parity, status,
-                               flag);
+        grid_refactor_call<NP>(src, b, n, HLq, Fq, lane, ob, logabs, phase, parity, status,
+                               LUFQHE_ST_FALLBACK);
       else
-        grid_refactor<NP>(src, b0 + q, n, HLq, Fq, lane, ob, logabs, phase, parity, status, flag);
+        grid_refactor<NP>(src, b, n, HLq, Fq, lane, ob, logabs, phase, parity, status,
+                          LUFQHE_ST_FALLBACK);
     }
   }
 }

@@ -1,5 +1,6 @@
 // Kernels of the mixed-precision batched complex LUP determinant, shared by
-// the complex128 (lup_mixed.cu) and complex64 (lup_mixed_c64.cu) entry points.
+// the complex128 (lup_mixed.cu), coordinate (lup_mixed_lll.cu) and complex64
+// (lup_mixed_c64.cu) entry points and by the CF call (cf.cu).
 //
 // Per matrix (one warp, shared memory), with FP64 used only where accuracy
 // needs it and almost all arithmetic on the FP32 and integer pipes, which on
@@ -61,6 +62,7 @@
 #include <type_traits>
 
 #include "bulk_copy.cuh"
+#include "lup_fp64_sub.cuh"
 #include "mixed_core.cuh"
 #include "mixed_grid.cuh"
 
@@ -258,10 +260,18 @@ __global__ void __launch_bounds__(kMaxWarpsMixed * 32)
 
 // The FP32 pass of the lane-grid path: each warp takes Grid::G consecutive
 // matrices at a time. NC = n for the register-tiled sizes, 0 for the generic
-// rule. DEFER: rejected matrices go to the call's pending list and (n = 24, 32)
-// the ones to refine to the saved matrices; else they are refined or
-// refactorised in FP64 right away, one at a time by the whole warp.
-template <int NP, int LPM, int NC, bool DEFER, class Src>
+// rule. FORM says where the matrices go that it does not accept:
+//  GRID_DEFER: to the call's pending list, and (n = 24, 32) those to refine to the
+//    saved matrices;
+//  GRID_INPLACE: refined or refactorised in FP64 right away, one at a time by the
+//    whole warp;
+//  GRID_ROUTED: so too, and the matrices that the policy routes to FP64
+//    (share64k; GRID_DEFER takes them as well) to the pending list, or, where a
+//    warp takes one matrix at a time, to FP64 right away. A form of its own, so
+//    that a call without a routed share runs none of its code (65536 LLL x n=16
+//    with one code for both: 669 us against 648).
+enum GridForm { GRID_INPLACE, GRID_ROUTED, GRID_DEFER };
+template <int NP, int LPM, int NC, int FORM, class Src>
 __global__ void __launch_bounds__(grid_warps(NP) * 32, grid_min_ctas(NP, NC))
     lup_mixed_grid_kernel(Src src, int n_rt, long long batch, float theta2,
                           unsigned int share64k, CallHead *head, unsigned int *pend, int refine,
@@ -270,6 +280,7 @@ __global__ void __launch_bounds__(grid_warps(NP) * 32, grid_min_ctas(NP, NC))
                           int8_t *__restrict__ parity, int32_t *__restrict__ status) {
   using Gd = Grid<NP, LPM>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr bool DEFER = FORM == GRID_DEFER;
   constexpr bool BULK = std::is_same<Src, DenseSource>::value;
   const int n = NC ? NC : n_rt;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -290,6 +301,18 @@ __global__ void __launch_bounds__(grid_warps(NP) * 32, grid_min_ctas(NP, NC))
   for (; u < units; u = nu, nu = u < units ? claim_matrix(head, lane, u) : units) {
     const long long b0 = u * Gd::G;
     const int cnt = (int)min((long long)Gd::G, batch - b0);
+    // a unit of routed matrices alone is not staged
+    if (FORM != GRID_INPLACE && share64k) {
+      const int grp = lane / Gd::LPM;
+      if (__all_sync(kFull, grp >= cnt || route_fp64_entry(src.first(b0 + grp, n), share64k))) {
+        if constexpr (DEFER || Gd::G > 1)
+          for (int q = 0; q < cnt; ++q) defer_fp64(head, pend, b0 + q, lane, true);
+        else
+          grid_refactor<NP>(src, b0, n, HLw, Fw, lane, b0, logabs, phase, parity, status,
+                            LUFQHE_ST_FP64);
+        continue;
+      }
+    }
     __syncwarp();
     bool staged = false;
     if constexpr (BULK) {
@@ -313,7 +336,8 @@ __global__ void __launch_bounds__(grid_warps(NP) * 32, grid_min_ctas(NP, NC))
     // substitution refined by the next pass, if the buffer has room; the others
     // are listed for FP64
     grid_unit<NP, LPM, NC, !DEFER, false>(
-        src, b0, b0, cnt, n, HLw, Fw, Iw, lane, theta2, share64k, refine != 0,
+        src, b0, b0, cnt, n, HLw, Fw, Iw, lane, theta2, FORM == GRID_ROUTED ? share64k : 0u,
+        refine != 0, [](int q) { return q; },
         [&](long long b, bool routed, bool can_refine, const CFF &prod, int exp_sum, int par) {
           if constexpr (NC != 0)
             if (can_refine && saved &&
@@ -579,6 +603,53 @@ __global__ void __launch_bounds__(kFallbackMaxWarps * 32)
   }
 }
 
+// The FP64 pass of the routed share at n <= 16 (LUFQHE_OPT_FP64_SHARE): the
+// listed matrices several per warp, as the plain kernels take them (lup_fp64_warp's
+// bits). In the FP32 pass, a warp per matrix between its units, they cost twice as
+// much and held up the other half of a unit (65536 x n=16, a quarter routed, us:
+// Gaussian 985 in place, 785 listed; n=8 361 and 196).
+template <int LPM, class Src>
+__global__ void __launch_bounds__(128)
+    lup_mixed_routed_kernel(Src src, int n, const CallHead *head, const unsigned int *pend,
+                            double *__restrict__ logabs, double *__restrict__ phase,
+                            int8_t *__restrict__ parity, int32_t *__restrict__ status) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int G = 32 / LPM;
+  const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int grp = lane / LPM, sub = lane % LPM, lds = n | 1;
+  const unsigned gmask = ((1u << LPM) - 1u) << (grp * LPM);
+  double2 *Mw = reinterpret_cast<double2 *>(smem_raw) + (size_t)warp * G * n * lds;
+  double2 *M = Mw + (size_t)grp * n * lds;
+  double *hold = reinterpret_cast<double *>(reinterpret_cast<double2 *>(smem_raw) +
+                                            (size_t)warps * G * n * lds) +
+                 (size_t)(warp * G + grp) * 2 * n;
+  const long long listed = head->pend_count;
+  const long long stride = (long long)gridDim.x * warps * G;
+  for (long long j0 = ((long long)blockIdx.x * warps + warp) * G; j0 < listed; j0 += stride) {
+    const int cnt = (int)min((long long)G, listed - j0);
+    const bool valid = grp < cnt;
+    const unsigned int b = valid ? pend[j0 + grp] & ~kPendRouted : 0u;
+    __syncwarp();
+    for (int q = 0; q < cnt; ++q)
+      load_rows(src, __shfl_sync(kFull, b, q * LPM), n, n, Mw + (size_t)q * n * lds, lds, n, lane);
+    __syncwarp();
+    int par = 0;
+    const int st = lup_fp64_sub<ARITH_FUSED, LPM>(M, lds, hold, n, sub, gmask, valid, &par);
+    double la, ph;
+    logdet_from_diag_sub<LPM>(M, lds, n, sub, valid && st == 0, par, &la, &ph);
+    if (!valid || sub != 0) continue;
+    if (st != 0) {
+      la = st == LUFQHE_ST_SINGULAR ? -INFINITY : NAN;
+      ph = st == LUFQHE_ST_SINGULAR ? 0.0 : NAN;
+      if (st != LUFQHE_ST_SINGULAR) par = 0;
+    }
+    logabs[b] = la;
+    if (phase) phase[b] = ph;
+    if (parity) parity[b] = (int8_t)par;
+    if (status) status[b] = st == LUFQHE_ST_NONFINITE ? st : st | LUFQHE_ST_FP64;
+  }
+}
+
 // the bulk-copy staging for complex128 matrices in device memory only
 inline int bulk_for(const DenseSource &s) { return g_bulk_loads && is_device_memory(s.A); }
 template <class S>
@@ -639,6 +710,23 @@ inline size_t fallback_smem_per_warp(int n) {
   return b;
 }
 
+// Shared-memory limit, and the grid of `warps`-warp CTAs over `units` units.
+template <class K>
+int grid_geometry(K kern, int warps, size_t smem, long long units, int *grid) {
+  int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)smem),
+                      "cudaFuncSetAttribute(mixed)");
+  if (rc) return rc;
+  int per_sm = 0;
+  rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, smem),
+                  "occupancy(mixed)");
+  if (rc) return rc;
+  const long long want = (units + warps - 1) / warps;
+  const long long cap = (long long)device_sm_count() * std::max(1, per_sm);
+  *grid = (int)std::min(want, cap);
+  return LUFQHE_SUCCESS;
+}
+
 template <class Src>
 int launch_fallback(Src src, int n, const CallHead *head, const unsigned int *pend,
                     long long batch, double *logabs, double *phase, int8_t *parity,
@@ -671,6 +759,22 @@ int launch_fallback(Src src, int n, const CallHead *head, const unsigned int *pe
   return check_cuda(cudaGetLastError(), "lup_mixed_fallback_kernel launch");
 }
 
+template <int LPM, class Src>
+int launch_routed(Src src, int n, const CallHead *head, const unsigned int *pend, long long batch,
+                  double *logabs, double *phase, int8_t *parity, int32_t *status,
+                  cudaStream_t stream) {
+  auto kern = lup_mixed_routed_kernel<LPM, Src>;
+  const int warps = sub_warps(n, LPM);
+  const size_t smem = sub_smem(n, LPM);
+  int grid = 0;
+  const int rc = grid_geometry(kern, warps, smem, (batch + 32 / LPM - 1) / (32 / LPM), &grid);
+  if (rc) return rc;
+  KernelTimer timer("lup_mixed_routed_kernel", n, stream);
+  kern<<<grid, warps * 32, smem, stream>>>(src, n, head, pend, logabs, phase, parity, status);
+  timer.stop();
+  return check_cuda(cudaGetLastError(), "lup_mixed_routed_kernel launch");
+}
+
 // The correction pass over a factor list of capacity cap (its length is
 // known only on the device): as many CTAs as fit, at most one per entry.
 template <int N, class Src, bool COPY>
@@ -696,23 +800,6 @@ int launch_fac_correct(Src src, const CallHead *head, const unsigned char *list,
                                                    status);
   timer.stop();
   return check_cuda(cudaGetLastError(), "lup_mixed_fac_correct_kernel launch");
-}
-
-// Shared-memory limit, and the grid of `warps`-warp CTAs over `units` units.
-template <class K>
-int grid_geometry(K kern, int warps, size_t smem, long long units, int *grid) {
-  int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem),
-                      "cudaFuncSetAttribute(mixed)");
-  if (rc) return rc;
-  int per_sm = 0;
-  rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, smem),
-                  "occupancy(mixed)");
-  if (rc) return rc;
-  const long long want = (units + warps - 1) / warps;
-  const long long cap = (long long)device_sm_count() * std::max(1, per_sm);
-  *grid = (int)std::min(want, cap);
-  return LUFQHE_SUCCESS;
 }
 
 // Warps per CTA of the in-place and finish kernels, in the tile layout.
@@ -765,7 +852,7 @@ template <int N, class Src>
 int launch_mixed_tile(Src src, long long batch, float theta2, double *logabs, double *phase,
                       int8_t *parity, int32_t *status, cudaStream_t stream) {
   using Gd = Grid<N, 32>;
-  auto kern = lup_mixed_grid_kernel<N, 32, N, true, Src>;
+  auto kern = lup_mixed_grid_kernel<N, 32, N, GRID_DEFER, Src>;
   auto fk = lup_mixed_finish_kernel<N, Src>;
   constexpr int gwarps = grid_warps(N);
   const size_t gsmem = Gd::kWarpBytes * gwarps;
@@ -803,20 +890,22 @@ int launch_mixed_tile(Src src, long long batch, float theta2, double *logabs, do
   return cs.release(stream, rc);
 }
 
-template <int NP, int LPM, int NC, bool DEFER, class Src>
+template <int NP, int LPM, int NC, int FORM, class Src>
 int launch_mixed_grid(Src src, int n, long long batch, float theta2, double *logabs,
                       double *phase, int8_t *parity, int32_t *status, cudaStream_t stream) {
   using Gd = Grid<NP, LPM>;
-  auto kern = lup_mixed_grid_kernel<NP, LPM, NC, DEFER, Src>;
+  auto kern = lup_mixed_grid_kernel<NP, LPM, NC, FORM, Src>;
   constexpr int warps = grid_warps(NP);
   const size_t smem = Gd::kWarpBytes * warps;
   const long long units = (batch + Gd::G - 1) / Gd::G;
   int grid = 0;
   int rc = grid_geometry(kern, warps, smem, units, &grid);
   if (rc) return rc;
+  // several matrices per warp: a routed share is listed
+  constexpr bool list = FORM == GRID_DEFER || (FORM == GRID_ROUTED && Gd::G > 1);
   CallState cs;
-  if (DEFER || needs_counter(units, (long long)grid * warps)) {
-    rc = cs.acquire(DEFER ? (size_t)batch : 0, 0, 0, stream);
+  if (list || needs_counter(units, (long long)grid * warps)) {
+    rc = cs.acquire(list ? (size_t)batch : 0, 0, 0, stream);
     if (rc) return cs.release(stream, rc);
   }
   {
@@ -828,25 +917,41 @@ int launch_mixed_grid(Src src, int n, long long batch, float theta2, double *log
     timer.stop();
   }
   rc = check_cuda(cudaGetLastError(), "lup_mixed_grid_kernel launch");
-  if constexpr (DEFER)
+  if constexpr (FORM == GRID_DEFER) {
     if (!rc)
       rc = launch_fallback(src, n, cs.head, cs.pend, batch, logabs, phase, parity, status, stream);
+  } else if constexpr (list) {
+    if (!rc)
+      rc = launch_routed<Gd::LPM / 2>(src, n, cs.head, cs.pend, batch, logabs, phase, parity,
+                                      status, stream);
+  }
   return cs.release(stream, rc);
 }
 
 // n <= 16: several matrices per warp, except in a batch of at most one matrix
 // per SM sub-partition, where a warp each has the least latency (64 LLL matrices
-// of n = 16: 23.2 us a call with two per warp, 18.7 us with one).
+// of n = 16: 23.2 us a call with two per warp, 18.7 us with one). With a routed
+// share a warp each up to two of the grid's strides, where the call then needs no
+// list (a tenth / half routed, us, a warp each | listed: 4096 x n=8 46/58 | 55/55,
+// n=16 83/113 | 111/111; listed 16384 x n=16 186/298, where the routed matrices
+// between the FP32 ones of a warp took 243/413).
 template <int NP, int NC, class Src>
 int launch_mixed_small(Src src, int n, long long batch, float theta2, double *logabs,
                        double *phase, int8_t *parity, int32_t *status, cudaStream_t stream) {
   constexpr int LPM = SmallGrid<NP>::LPM;
   constexpr int NP1 = NP == 12 ? 16 : NP;  // whole 8-column slots
+  if (fp64_share_64k(n) != 0) {
+    if (batch <= 32ll * device_sm_count())
+      return launch_mixed_grid<NP1, 32, NC, GRID_ROUTED>(src, n, batch, theta2, logabs, phase,
+                                                         parity, status, stream);
+    return launch_mixed_grid<NP, LPM, NC, GRID_ROUTED>(src, n, batch, theta2, logabs, phase,
+                                                       parity, status, stream);
+  }
   if (batch <= 4ll * device_sm_count())
-    return launch_mixed_grid<NP1, 32, NC, false>(src, n, batch, theta2, logabs, phase, parity,
-                                                 status, stream);
-  return launch_mixed_grid<NP, LPM, NC, false>(src, n, batch, theta2, logabs, phase, parity,
-                                               status, stream);
+    return launch_mixed_grid<NP1, 32, NC, GRID_INPLACE>(src, n, batch, theta2, logabs, phase,
+                                                        parity, status, stream);
+  return launch_mixed_grid<NP, LPM, NC, GRID_INPLACE>(src, n, batch, theta2, logabs, phase,
+                                                      parity, status, stream);
 }
 
 // Sources whose matrices are always of odd order (CF matrices, n = 2Q + 3)
@@ -892,8 +997,8 @@ int launch_mixed_src(Src src, int n, long long batch, double *logabs, double *ph
       default: return launch_mixed_small<16, 0>(src, n, batch, th2, logabs, phase, parity, status, stream);
     }
   }
-  if (n <= 24) return launch_mixed_grid<24, 32, 0, true>(src, n, batch, th2, logabs, phase, parity, status, stream);
-  if (n <= 32) return launch_mixed_grid<32, 32, 0, true>(src, n, batch, th2, logabs, phase, parity, status, stream);
+  if (n <= 24) return launch_mixed_grid<24, 32, 0, GRID_DEFER>(src, n, batch, th2, logabs, phase, parity, status, stream);
+  if (n <= 32) return launch_mixed_grid<32, 32, 0, GRID_DEFER>(src, n, batch, th2, logabs, phase, parity, status, stream);
   const size_t per_warp = mixed_smem_per_warp(n);
   const size_t optin = device_smem_optin();
   int warps = (int)(optin / per_warp);

@@ -802,13 +802,15 @@ int launch_fac_correct(Src src, const CallHead *head, const unsigned char *list,
   return check_cuda(cudaGetLastError(), "lup_mixed_fac_correct_kernel launch");
 }
 
-// Warps per CTA of the in-place and finish kernels, in the tile layout.
+// Warps per CTA of a register-tiled size's kernel that takes up to `most` (option 2).
+inline int tuned_warps(int most) {
+  return g_tile_warps > 0 && g_tile_warps < most ? g_tile_warps : most;
+}
+// The same of the in-place and finish kernels, in the tile layout.
 template <int N>
 int tile_warps() {
-  int warps = (int)(device_smem_optin() / tile_smem_per_warp<N>());
-  int cap = tile_max_warps(N);
-  if (g_tile_warps > 0 && g_tile_warps < cap) cap = g_tile_warps;
-  return std::min(warps, cap);
+  return std::min((int)(device_smem_optin() / tile_smem_per_warp<N>()),
+                  tuned_warps(tile_max_warps(N)));
 }
 // Room for `share` of a batch.
 inline long long share_cap(double share, long long batch) {
@@ -854,7 +856,7 @@ int launch_mixed_tile(Src src, long long batch, float theta2, double *logabs, do
   using Gd = Grid<N, 32>;
   auto kern = lup_mixed_grid_kernel<N, 32, N, GRID_DEFER, Src>;
   auto fk = lup_mixed_finish_kernel<N, Src>;
-  constexpr int gwarps = grid_warps(N);
+  const int gwarps = tuned_warps(grid_warps(N));
   const size_t gsmem = Gd::kWarpBytes * gwarps;
   const int fwarps = tile_warps<N>();
   const size_t fsmem = tile_smem_per_warp<N>() * fwarps;
@@ -895,7 +897,7 @@ int launch_mixed_grid(Src src, int n, long long batch, float theta2, double *log
                       double *phase, int8_t *parity, int32_t *status, cudaStream_t stream) {
   using Gd = Grid<NP, LPM>;
   auto kern = lup_mixed_grid_kernel<NP, LPM, NC, FORM, Src>;
-  constexpr int warps = grid_warps(NP);
+  const int warps = NC ? tuned_warps(grid_warps(NP)) : grid_warps(NP);
   const size_t smem = Gd::kWarpBytes * warps;
   const long long units = (batch + Gd::G - 1) / Gd::G;
   int grid = 0;

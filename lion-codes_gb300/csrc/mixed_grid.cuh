@@ -775,9 +775,9 @@ __device__ __noinline__ void grid_refactor_call(const Src src, long long sb, int
 // HLw + q kHL, into outputs ob0 + at(q): the FP32 path, then what it does not
 // accept: refined or refactorised right here (INPLACE, n <= 16), or handed to
 // defer(b, routed, can_refine, prod, exp_sum, par). share64k: the share routed to
-// FP64, of which several matrices per warp may hold a part: they go to defer in
-// any case (the kernels ask for units of such matrices alone before they stage
-// them). CALL: FP64 out of line.
+// FP64, for units that hold some of it beside others: it goes to defer in any case
+// (the kernels ask for units of such matrices alone before they stage them). CALL:
+// FP64 out of line.
 template <int NP, int LPM, int NC, bool INPLACE, bool CALL, class Src, class At, class Defer>
 __device__ __forceinline__ void grid_unit(const Src &src, long long b0, long long ob0, int cnt,
                                           int n, float4 *HLw, float2 *Fw, int *Iw, int lane,
@@ -792,7 +792,7 @@ __device__ __forceinline__ void grid_unit(const Src &src, long long b0, long lon
   int code = grid_factor<NP, LPM, NC>(HLw + grp * Gd::kHL, Fw + grp * Gd::kF, Iw + grp * 2 * NP, n,
                                       lane, theta2, prod, exp_sum, corr, par);
   bool routed = false;
-  if (Gd::G > 1 && share64k && grp < cnt && code != TILE_NONFINITE) {
+  if (share64k && grp < cnt && code != TILE_NONFINITE) {
     routed = route_fp64_entry(src.first(b0 + grp, n), share64k);
     if (routed) code = TILE_REJECT;
   }
@@ -818,7 +818,7 @@ __device__ __forceinline__ void grid_unit(const Src &src, long long b0, long lon
       emit_nonfinite(lane, ob, logabs, phase, parity, status);
       continue;
     }
-    const bool rt = Gd::G > 1 && share64k && __shfl_sync(kFull, (int)routed, from) != 0;
+    const bool rt = Gd::G > 1 ? share64k && __shfl_sync(kFull, (int)routed, from) != 0 : routed;
     if constexpr (!INPLACE) {
       defer(b, rt, cq == TILE_REFINE && refine, pq, eq, rq);
     } else if (rt) {

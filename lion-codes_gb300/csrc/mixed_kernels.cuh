@@ -265,12 +265,18 @@ __global__ void __launch_bounds__(kMaxWarpsMixed * 32)
 //    saved matrices;
 //  GRID_INPLACE: refined or refactorised in FP64 right away, one at a time by the
 //    whole warp;
-//  GRID_ROUTED: so too, and the matrices that the policy routes to FP64
-//    (share64k; GRID_DEFER takes them as well) to the pending list, or, where a
-//    warp takes one matrix at a time, to FP64 right away. A form of its own, so
-//    that a call without a routed share runs none of its code (65536 LLL x n=16
-//    with one code for both: 669 us against 648).
-enum GridForm { GRID_INPLACE, GRID_ROUTED, GRID_DEFER };
+//  .._ROUTED: so too, and the matrices that the policy routes to FP64 (share64k) to
+//    the pending list, or, in place where a warp takes one matrix at a time, to FP64
+//    right away. Forms of their own, so that a call without a routed share runs
+//    none of that code (with one code for both: 65536 LLL x n=16 669 us against 648,
+//    8192 LLL x n=27 750 against 704). GRID_DEFER keeps grid_unit's own look at the
+//    share, which never finds one there: without it the compiler's schedule of the
+//    padded n = 25..31 is 4% slower (8192 Gaussian x n=27 430 us against 416).
+enum GridForm { GRID_INPLACE, GRID_INPLACE_ROUTED, GRID_DEFER, GRID_DEFER_ROUTED };
+constexpr bool grid_defers(int form) { return form == GRID_DEFER || form == GRID_DEFER_ROUTED; }
+constexpr bool grid_routes(int form) {
+  return form == GRID_INPLACE_ROUTED || form == GRID_DEFER_ROUTED;
+}
 template <int NP, int LPM, int NC, int FORM, class Src>
 __global__ void __launch_bounds__(grid_warps(NP) * 32, grid_min_ctas(NP, NC))
     lup_mixed_grid_kernel(Src src, int n_rt, long long batch, float theta2,
@@ -280,7 +286,7 @@ __global__ void __launch_bounds__(grid_warps(NP) * 32, grid_min_ctas(NP, NC))
                           int8_t *__restrict__ parity, int32_t *__restrict__ status) {
   using Gd = Grid<NP, LPM>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr bool DEFER = FORM == GRID_DEFER;
+  constexpr bool DEFER = grid_defers(FORM);
   constexpr bool BULK = std::is_same<Src, DenseSource>::value;
   const int n = NC ? NC : n_rt;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -302,7 +308,7 @@ __global__ void __launch_bounds__(grid_warps(NP) * 32, grid_min_ctas(NP, NC))
     const long long b0 = u * Gd::G;
     const int cnt = (int)min((long long)Gd::G, batch - b0);
     // a unit of routed matrices alone is not staged
-    if (FORM != GRID_INPLACE && share64k) {
+    if (grid_routes(FORM) && share64k) {
       const int grp = lane / Gd::LPM;
       if (__all_sync(kFull, grp >= cnt || route_fp64_entry(src.first(b0 + grp, n), share64k))) {
         if constexpr (DEFER || Gd::G > 1)
@@ -336,8 +342,9 @@ __global__ void __launch_bounds__(grid_warps(NP) * 32, grid_min_ctas(NP, NC))
     // substitution refined by the next pass, if the buffer has room; the others
     // are listed for FP64
     grid_unit<NP, LPM, NC, !DEFER, false>(
-        src, b0, b0, cnt, n, HLw, Fw, Iw, lane, theta2, FORM == GRID_ROUTED ? share64k : 0u,
-        refine != 0, [](int q) { return q; },
+        src, b0, b0, cnt, n, HLw, Fw, Iw, lane, theta2,
+        FORM == GRID_INPLACE || (!DEFER && Gd::G == 1) ? 0u : share64k, refine != 0,
+        [](int q) { return q; },
         [&](long long b, bool routed, bool can_refine, const CFF &prod, int exp_sum, int par) {
           if constexpr (NC != 0)
             if (can_refine && saved &&
@@ -854,7 +861,8 @@ template <int N, class Src>
 int launch_mixed_tile(Src src, long long batch, float theta2, double *logabs, double *phase,
                       int8_t *parity, int32_t *status, cudaStream_t stream) {
   using Gd = Grid<N, 32>;
-  auto kern = lup_mixed_grid_kernel<N, 32, N, GRID_DEFER, Src>;
+  auto kern = fp64_share_64k(N) ? lup_mixed_grid_kernel<N, 32, N, GRID_DEFER_ROUTED, Src>
+                                : lup_mixed_grid_kernel<N, 32, N, GRID_DEFER, Src>;
   auto fk = lup_mixed_finish_kernel<N, Src>;
   const int gwarps = tuned_warps(grid_warps(N));
   const size_t gsmem = Gd::kWarpBytes * gwarps;
@@ -904,7 +912,7 @@ int launch_mixed_grid(Src src, int n, long long batch, float theta2, double *log
   int rc = grid_geometry(kern, warps, smem, units, &grid);
   if (rc) return rc;
   // several matrices per warp: a routed share is listed
-  constexpr bool list = FORM == GRID_DEFER || (FORM == GRID_ROUTED && Gd::G > 1);
+  constexpr bool list = grid_defers(FORM) || (grid_routes(FORM) && Gd::G > 1);
   CallState cs;
   if (list || needs_counter(units, (long long)grid * warps)) {
     rc = cs.acquire(list ? (size_t)batch : 0, 0, 0, stream);
@@ -919,7 +927,7 @@ int launch_mixed_grid(Src src, int n, long long batch, float theta2, double *log
     timer.stop();
   }
   rc = check_cuda(cudaGetLastError(), "lup_mixed_grid_kernel launch");
-  if constexpr (FORM == GRID_DEFER) {
+  if constexpr (grid_defers(FORM)) {
     if (!rc)
       rc = launch_fallback(src, n, cs.head, cs.pend, batch, logabs, phase, parity, status, stream);
   } else if constexpr (list) {
@@ -944,16 +952,27 @@ int launch_mixed_small(Src src, int n, long long batch, float theta2, double *lo
   constexpr int NP1 = NP == 12 ? 16 : NP;  // whole 8-column slots
   if (fp64_share_64k(n) != 0) {
     if (batch <= 32ll * device_sm_count())
-      return launch_mixed_grid<NP1, 32, NC, GRID_ROUTED>(src, n, batch, theta2, logabs, phase,
-                                                         parity, status, stream);
-    return launch_mixed_grid<NP, LPM, NC, GRID_ROUTED>(src, n, batch, theta2, logabs, phase,
-                                                       parity, status, stream);
+      return launch_mixed_grid<NP1, 32, NC, GRID_INPLACE_ROUTED>(src, n, batch, theta2, logabs,
+                                                                 phase, parity, status, stream);
+    return launch_mixed_grid<NP, LPM, NC, GRID_INPLACE_ROUTED>(src, n, batch, theta2, logabs,
+                                                               phase, parity, status, stream);
   }
   if (batch <= 4ll * device_sm_count())
     return launch_mixed_grid<NP1, 32, NC, GRID_INPLACE>(src, n, batch, theta2, logabs, phase,
                                                         parity, status, stream);
   return launch_mixed_grid<NP, LPM, NC, GRID_INPLACE>(src, n, batch, theta2, logabs, phase,
                                                       parity, status, stream);
+}
+
+// 17 <= n <= 31 without a register-tiled rule, padded to NP.
+template <int NP, class Src>
+int launch_mixed_padded(Src src, int n, long long batch, float theta2, double *logabs,
+                        double *phase, int8_t *parity, int32_t *status, cudaStream_t stream) {
+  if (fp64_share_64k(n))
+    return launch_mixed_grid<NP, 32, 0, GRID_DEFER_ROUTED>(src, n, batch, theta2, logabs, phase,
+                                                           parity, status, stream);
+  return launch_mixed_grid<NP, 32, 0, GRID_DEFER>(src, n, batch, theta2, logabs, phase, parity,
+                                                  status, stream);
 }
 
 // Sources whose matrices are always of odd order (CF matrices, n = 2Q + 3)
@@ -999,8 +1018,8 @@ int launch_mixed_src(Src src, int n, long long batch, double *logabs, double *ph
       default: return launch_mixed_small<16, 0>(src, n, batch, th2, logabs, phase, parity, status, stream);
     }
   }
-  if (n <= 24) return launch_mixed_grid<24, 32, 0, GRID_DEFER>(src, n, batch, th2, logabs, phase, parity, status, stream);
-  if (n <= 32) return launch_mixed_grid<32, 32, 0, GRID_DEFER>(src, n, batch, th2, logabs, phase, parity, status, stream);
+  if (n <= 24) return launch_mixed_padded<24>(src, n, batch, th2, logabs, phase, parity, status, stream);
+  if (n <= 32) return launch_mixed_padded<32>(src, n, batch, th2, logabs, phase, parity, status, stream);
   const size_t per_warp = mixed_smem_per_warp(n);
   const size_t optin = device_smem_optin();
   int warps = (int)(optin / per_warp);

@@ -287,7 +287,7 @@ __device__ void small_item(const WorkItem &w, unsigned char *base, int lane, flo
     }
     for (; w.share64k && cnt < Gd::G && j < w.count; ++j) {
       if (route_fp64_entry(src.first(w.first + j, n), w.share64k)) {
-        grid_refactor_call<NP>(src, w.first + j, n, HLw, Fw, lane, w.out + j, logabs, phase,
+        grid_refactor_call<NP>(src, w.first + j, n, HLw, Fw, Iw, lane, w.out + j, logabs, phase,
                                parity, status, LUFQHE_ST_FP64);
       } else {
         if (cnt == lane / Gd::LPM) mine = j;

@@ -749,31 +749,33 @@ __device__ __forceinline__ void repack_f(float2 *F, int lane) {
 }
 
 // FP64 refactorisation of matrix sb of src into output ob, in one matrix's area
-// of the lane grid, by the whole warp. Sizes up to 16 have no correction, so the
-// row scales may lie over F where no padding is left after the matrix (n = NP).
+// of the lane grid, by the whole warp. The row scales lie in the padding after the
+// matrix, or, where there is none (n = NP = 8, 12, 16: sizes without a correction),
+// over F; the correction of n >= 17 takes F and the ints.
 template <int NP, class Src>
 __device__ __forceinline__ void grid_refactor(const Src &src, long long sb, int n, float4 *HL,
-                                              float2 *F, int lane, long long ob, double *logabs,
-                                              double *phase, int8_t *parity, int32_t *status,
-                                              int flag) {
+                                              float2 *F, int *ints, int lane, long long ob,
+                                              double *logabs, double *phase, int8_t *parity,
+                                              int32_t *status, int flag) {
   double *hold = n < NP ? reinterpret_cast<double *>(HL + (size_t)n * (n + 1))
                         : reinterpret_cast<double *>(F);
+  const CorrScratch cs{F, ints, hold};
   fallback_fp64_src(src, sb, n, reinterpret_cast<double2 *>(HL), n + 1, hold, lane, ob, logabs,
-                    phase, parity, status, flag);
+                    phase, parity, status, flag, NP > 16 ? &cs : nullptr);
 }
 // The same out of line, for a kernel with many sizes. (In the batched kernels
 // the call cost more than the code it saves: 65536 LLL x n=16 645 -> 677 us.)
 template <int NP, class Src>
 __device__ __noinline__ void grid_refactor_call(const Src src, long long sb, int n, float4 *HL,
-                                                float2 *F, int lane, long long ob, double *logabs,
-                                                double *phase, int8_t *parity, int32_t *status,
-                                                int flag) {
-  grid_refactor<NP>(src, sb, n, HL, F, lane, ob, logabs, phase, parity, status, flag);
+                                                float2 *F, int *ints, int lane, long long ob,
+                                                double *logabs, double *phase, int8_t *parity,
+                                                int32_t *status, int flag) {
+  grid_refactor<NP>(src, sb, n, HL, F, ints, lane, ob, logabs, phase, parity, status, flag);
 }
 
 // One unit of a warp: matrices b0 + at(q), q < cnt, of src, staged in areas
 // HLw + q kHL, into outputs ob0 + at(q): the FP32 path, then what it does not
-// accept: refined or refactorised right here (INPLACE, n <= 16), or handed to
+// accept: refined or refactorised right here (INPLACE, NP < 32), or handed to
 // defer(b, routed, can_refine, prod, exp_sum, par). share64k: the share routed to
 // FP64, for units that hold some of it beside others: it goes to defer in any case
 // (the kernels ask for units of such matrices alone before they stage them). CALL:
@@ -826,12 +828,13 @@ __device__ __forceinline__ void grid_unit(const Src &src, long long b0, long lon
     } else {
       float4 *HLq = HLw + q * Gd::kHL;
       float2 *Fq = Fw + q * Gd::kF;
+      int *Iq = Iw + q * 2 * NP;
       if constexpr (NC != 0) {
         if (cq == TILE_REFINE && refine) {
           float2 *Rm = reinterpret_cast<float2 *>(HLq);
           repack_f<NP, NC>(Fq, lane);
           if (mixed_refine_tile<NC>(Fq, Rm, Rm + NC * (NC + 1),
-                                    reinterpret_cast<float2 *>(Iw + q * 2 * NP), lane, theta2,
+                                    reinterpret_cast<float2 *>(Iq), lane, theta2,
                                     tile_la_est(pq, eq), kq)) {
             out.push(lane, ob, pq, eq, kq, rq, logabs, phase, parity, status);
             continue;
@@ -839,10 +842,10 @@ __device__ __forceinline__ void grid_unit(const Src &src, long long b0, long lon
         }
       }
       if constexpr (CALL)
-        grid_refactor_call<NP>(src, b, n, HLq, Fq, lane, ob, logabs, phase, parity, status,
+        grid_refactor_call<NP>(src, b, n, HLq, Fq, Iq, lane, ob, logabs, phase, parity, status,
                                LUFQHE_ST_FALLBACK);
       else
-        grid_refactor<NP>(src, b, n, HLq, Fq, lane, ob, logabs, phase, parity, status,
+        grid_refactor<NP>(src, b, n, HLq, Fq, Iq, lane, ob, logabs, phase, parity, status,
                           LUFQHE_ST_FALLBACK);
     }
   }

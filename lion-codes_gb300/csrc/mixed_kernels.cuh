@@ -118,6 +118,11 @@ __device__ __forceinline__ long long claim_matrix(CallHead *head, int lane, long
 constexpr unsigned int kPendRouted = 0x80000000u;
 
 constexpr int kDeferMinN = 24;
+// Matrices per SM up to which a batch of 17 <= n <= 23 refactorises in place: one
+// launch and no state block (64 Gaussian matrices of n = 20: 39.0 us with a second
+// kernel, 35.5 in place; 500 LLL 147, 136; 1000 LLL 160, 150). Beyond that the
+// rejected matrices of an SM wait for one another (2280 LLL: 176 listed, 196).
+constexpr long long kInplaceMaxPerSm = 8;
 // The same of the lane-grid kernels: shared memory holds 16 warps an SM at
 // NP = 16 (13.5 KB each), 15 at 24 (14.8 KB) and 8 at 32 (25.7 KB).
 constexpr int grid_warps(int np) { return np == 24 ? 3 : 4; }
@@ -280,9 +285,9 @@ constexpr bool grid_routes(int form) {
 template <int NP, int LPM, int NC, int FORM, class Src>
 __global__ void __launch_bounds__(grid_warps(NP) * 32, grid_min_ctas(NP, NC))
     lup_mixed_grid_kernel(Src src, int n_rt, long long batch, float theta2,
-                          unsigned int share64k, CallHead *head, unsigned int *pend, int refine,
-                          unsigned char *saved, long long saved_cap, int bulk,
-                          double *__restrict__ logabs, double *__restrict__ phase,
+                          unsigned int share64k, CallHead *claims, CallHead *head,
+                          unsigned int *pend, int refine, unsigned char *saved, long long saved_cap,
+                          int bulk, double *__restrict__ logabs, double *__restrict__ phase,
                           int8_t *__restrict__ parity, int32_t *__restrict__ status) {
   using Gd = Grid<NP, LPM>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -302,9 +307,9 @@ __global__ void __launch_bounds__(grid_warps(NP) * 32, grid_min_ctas(NP, NC))
 
   DeferredOut out;
   const long long units = (batch + Gd::G - 1) / Gd::G;
-  long long u = claim_matrix(head, lane, -1);
-  long long nu = u < units ? claim_matrix(head, lane, u) : units;
-  for (; u < units; u = nu, nu = u < units ? claim_matrix(head, lane, u) : units) {
+  long long u = claim_matrix(claims, lane, -1);
+  long long nu = u < units ? claim_matrix(claims, lane, u) : units;
+  for (; u < units; u = nu, nu = u < units ? claim_matrix(claims, lane, u) : units) {
     const long long b0 = u * Gd::G;
     const int cnt = (int)min((long long)Gd::G, batch - b0);
     // a unit of routed matrices alone is not staged
@@ -314,7 +319,7 @@ __global__ void __launch_bounds__(grid_warps(NP) * 32, grid_min_ctas(NP, NC))
         if constexpr (DEFER || Gd::G > 1)
           for (int q = 0; q < cnt; ++q) defer_fp64(head, pend, b0 + q, lane, true);
         else
-          grid_refactor<NP>(src, b0, n, HLw, Fw, lane, b0, logabs, phase, parity, status,
+          grid_refactor<NP>(src, b0, n, HLw, Fw, Iw, lane, b0, logabs, phase, parity, status,
                             LUFQHE_ST_FP64);
         continue;
       }
@@ -703,8 +708,8 @@ struct CallState {
 };
 
 // Whether warps must claim matrices from a counter: a batch beyond two strides
-// of the grid. (A call that takes a state block anyway, for its pending list
-// or host-link copies, claims from the block's zeroed counter regardless.)
+// of the grid. (The calls at n = 24 and 32, which take a state block anyway, and
+// those above 32 claim from the block's zeroed counter regardless.)
 inline bool needs_counter(long long batch, long long grid_warps) {
   return batch > 2 * grid_warps;
 }
@@ -882,8 +887,9 @@ int launch_mixed_tile(Src src, long long batch, float theta2, double *logabs, do
   {
     KernelTimer timer("lup_mixed_tile_kernel", N, stream);
     kern<<<grid, gwarps * 32, gsmem, stream>>>(src, N, batch, theta2, fp64_share_64k(N), cs.head,
-                                               cs.pend, g_mixed_refine, cs.refine, refine_cap,
-                                               bulk_for(src), logabs, phase, parity, status);
+                                               cs.head, cs.pend, g_mixed_refine, cs.refine,
+                                               refine_cap, bulk_for(src), logabs, phase, parity,
+                                               status);
     timer.stop();
   }
   rc = check_cuda(cudaGetLastError(), "lup_mixed_grid_kernel launch");
@@ -913,17 +919,21 @@ int launch_mixed_grid(Src src, int n, long long batch, float theta2, double *log
   if (rc) return rc;
   // several matrices per warp: a routed share is listed
   constexpr bool list = grid_defers(FORM) || (grid_routes(FORM) && Gd::G > 1);
+  // (a list alone does not make the warps claim: within two strides the first
+  // ones to claim sat together on few SMs, 3000 x n=17 87 us by stride, 119 claimed)
+  const bool counter = needs_counter(units, (long long)grid * warps);
   CallState cs;
-  if (list || needs_counter(units, (long long)grid * warps)) {
+  if (list || counter) {
     rc = cs.acquire(list ? (size_t)batch : 0, 0, 0, stream);
     if (rc) return cs.release(stream, rc);
   }
   {
     // (recorded under the names of the two rules)
     KernelTimer timer(NC ? "lup_mixed_tile_kernel" : "lup_mixed_kernel", n, stream);
-    kern<<<grid, warps * 32, smem, stream>>>(src, n, batch, theta2, fp64_share_64k(n), cs.head,
-                                             cs.pend, g_mixed_refine, nullptr, 0, bulk_for(src),
-                                             logabs, phase, parity, status);
+    kern<<<grid, warps * 32, smem, stream>>>(src, n, batch, theta2, fp64_share_64k(n),
+                                             counter ? cs.head : nullptr, cs.head, cs.pend,
+                                             g_mixed_refine, nullptr, 0, bulk_for(src), logabs,
+                                             phase, parity, status);
     timer.stop();
   }
   rc = check_cuda(cudaGetLastError(), "lup_mixed_grid_kernel launch");
@@ -964,10 +974,15 @@ int launch_mixed_small(Src src, int n, long long batch, float theta2, double *lo
                                                       parity, status, stream);
 }
 
-// 17 <= n <= 31 without a register-tiled rule, padded to NP.
+// 17 <= n <= 31 without a register-tiled rule, padded to NP; the smaller of them in
+// place in small batches.
 template <int NP, class Src>
 int launch_mixed_padded(Src src, int n, long long batch, float theta2, double *logabs,
                         double *phase, int8_t *parity, int32_t *status, cudaStream_t stream) {
+  if constexpr (NP == 24)
+    if (batch <= kInplaceMaxPerSm * device_sm_count())
+      return launch_mixed_grid<NP, 32, 0, GRID_INPLACE_ROUTED>(src, n, batch, theta2, logabs, phase,
+                                                               parity, status, stream);
   if (fp64_share_64k(n))
     return launch_mixed_grid<NP, 32, 0, GRID_DEFER_ROUTED>(src, n, batch, theta2, logabs, phase,
                                                            parity, status, stream);

@@ -454,9 +454,9 @@ struct NamedBarrier {
 // lane) while the others exchange the rows: 3 barriers per column instead of 7,
 // and no search or division repeated on several warps. The columns take the
 // warps in turn, so that the SM sub-partitions share that work. us, before ->
-// now, fused / reference arithmetic: 2048 LLL x n=64 (6 warps) 1724 -> 1620 /
-// 3607 -> 3355, 4096 x n=48 1469 -> 1424 / 3326 -> 2968; the FP64 pipe is 80 to
-// 88% busy. `red` is at least 2 words of shared scratch; tid and nthr number the
+// now, fused / reference arithmetic: 2048 LLL x n=64 (6 warps) 1724 -> 1588 /
+// 3602 -> 3345, 4096 x n=48 1469 -> 1376 / 3317 -> 2969, 1900 x n=33 300 -> 277 /
+// 698 -> 575; the FP64 pipe is the bound. `red` is at least 2 words of shared scratch; tid and nthr number the
 // group's threads (two warps or more). Group-uniform return value and parity.
 template <int ARITH, class Bar = CtaBarrier>
 __device__ int lup_fp64_group(double2 *M, int lds, double *hold, int n, int tid, int nthr,
@@ -573,12 +573,6 @@ __device__ int lup_fp64_group(double2 *M, int lds, double *hold, int n, int tid,
     if (j == n - 1) break;
     if (warp == lead) {
       const double2 piv = M[p * lds + j], top = M[j * lds + j];
-      double2 a[2];
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int i = j + 1 + lane + 32 * q;
-        a[q] = i == p ? top : i < n ? M[i * lds + j] : make_double2(0.0, 0.0);
-      }
       __syncwarp();
       if (lane == 0) M[j * lds + j] = piv;
       const double den = pivot_den<ARITH>(piv);
@@ -589,19 +583,19 @@ __device__ int lup_fp64_group(double2 *M, int lds, double *hold, int n, int tid,
         const long long db = abs_bits(den);
         den_safe = db >= 0x03f0000000000000ll && db <= 0x7bf0000000000000ll;  // [2^-960, 2^960]
       }
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int i = j + 1 + lane + 32 * q;
-        if (j + 1 + 32 * q >= n) continue;
-        if (i < n) {
-          if (ARITH == ARITH_REF) {
-            const double nx = __dadd_rn(__dmul_rn(a[q].x, piv.x), __dmul_rn(a[q].y, piv.y));
-            const double ny = __dsub_rn(__dmul_rn(a[q].y, piv.x), __dmul_rn(a[q].x, piv.y));
-            M[i * lds + j] = make_double2(div_rn_markstein(nx, den, y, den_safe),
-                                          div_rn_markstein(ny, den, y, den_safe));
-          } else {
-            M[i * lds + j] = cdiv_pivot<ARITH>(a[q], piv, den);
-          }
+      // (a loop: unrolled, the second round's arithmetic was issued under a false
+      // predicate in every column with at most 32 rows below: 1000 x n=33 161 us
+      // against 146)
+#pragma unroll 1
+      for (int i = j + 1 + lane; i < n; i += 32) {
+        const double2 a = i == p ? top : M[i * lds + j];
+        if (ARITH == ARITH_REF) {
+          const double nx = __dadd_rn(__dmul_rn(a.x, piv.x), __dmul_rn(a.y, piv.y));
+          const double ny = __dsub_rn(__dmul_rn(a.y, piv.x), __dmul_rn(a.x, piv.y));
+          M[i * lds + j] = make_double2(div_rn_markstein(nx, den, y, den_safe),
+                                        div_rn_markstein(ny, den, y, den_safe));
+        } else {
+          M[i * lds + j] = cdiv_pivot<ARITH>(a, piv, den);
         }
       }
     }
@@ -611,22 +605,9 @@ __device__ int lup_fp64_group(double2 *M, int lds, double *hold, int n, int tid,
     double2 *T = M + (j + 1) * lds + j + 1;
     const double2 *L = M + (j + 1) * lds + j, *U = M + j * lds + j + 1;
     StrideWalk w(tid, nthr, m);
-    for (int e = tid; e < mm; e += 2 * nthr) {
-      const int i0 = w.i, k0 = w.k;
+    for (int e = tid; e < mm; e += nthr) {
+      T[w.i * lds + w.k] = cmsub<ARITH>(T[w.i * lds + w.k], L[w.i * lds], U[w.k]);
       w.next(m);
-      const int i1 = w.i, k1 = w.k;
-      w.next(m);
-      if (e - lane + nthr < mm) {  // warp-uniform: two entries, one's loads over the other's work
-        const bool on = e + nthr < mm;
-        const int f1 = on ? i1 * lds + k1 : 0;
-        const double2 s0 = T[i0 * lds + k0], l0 = L[i0 * lds], u0 = U[k0];
-        const double2 s1 = T[f1], l1 = L[on ? i1 * lds : 0], u1 = U[on ? k1 : 0];
-        const double2 r0 = cmsub<ARITH>(s0, l0, u0), r1 = cmsub<ARITH>(s1, l1, u1);
-        T[i0 * lds + k0] = r0;
-        if (on) T[f1] = r1;
-      } else {
-        T[i0 * lds + k0] = cmsub<ARITH>(T[i0 * lds + k0], L[i0 * lds], U[k0]);
-      }
     }
     bar.sync();
   }

@@ -210,12 +210,14 @@ __global__ void write_det_kernel(T *A, int n, int lda, long long batch,
 // n > 32: one matrix per CTA of group_warps(n) warps (lup_fp64_group). With one
 // warp per matrix an SM holds only the 3-4 matrices its shared memory fits
 // (n=64: 66 KB each), too few warps to cover the FP64 pipe's latency.
-constexpr int kGroupMaxWarps = 6;
+constexpr int kGroupMaxWarps = 6, kGroupMinCtas = 6;
 constexpr int kGroupMinN = kFp64GroupMinN;
 // 4 warps up to n = 48, 6 above, where an SM holds 3 or 4 matrices only (2048
-// LLL x n=64, fused, us with 4 / 5 / 6 / 8 warps: 1745 / 1620 / 1621 / 1615;
-// reference arithmetic 3592 / 3395 / 3354 / 3410; 4096 x n=48 fused 1424 / 1425 /
-// 1431 / 1471).
+// LLL x n=64, us with 4 / 5 / 6 / 8 warps, when the multipliers of a column were
+// unrolled: fused 1745 / 1620 / 1621 / 1615, now 1588 with 6; reference arithmetic
+// 3592 / 3395 / 3354 / 3410; 4096 x n=48 fused 1424 / 1425 / 1431 / 1471, now 1376
+// with 4). Compiled for 56 registers, 9 CTAs of 4 warps (with 60, 2000 x n=36 in
+// reference arithmetic took 768 us instead of 716).
 constexpr int kWarpMaxN = 40;
 constexpr int group_warps(int n) { return n > 48 ? kGroupMaxWarps : kFp64GroupWarps; }
 
@@ -223,7 +225,7 @@ constexpr int group_warps(int n) { return n > 48 ? kGroupMaxWarps : kFp64GroupWa
 // extended-precision correction (fp64_correct_group; its scratch follows the
 // row scales in shared memory).
 template <int ARITH, class Src, class Out = double2, bool CORRECT = false>
-__global__ void __launch_bounds__(kGroupMaxWarps * 32)
+__global__ void __launch_bounds__(kGroupMaxWarps * 32, kGroupMinCtas)
     lup_plain_group_kernel(Src src, Out *__restrict__ Aout, int n, int lda, long long batch,
                            double *__restrict__ logabs, double *__restrict__ phase,
                            int8_t *__restrict__ parity, int32_t *__restrict__ status,
@@ -334,16 +336,18 @@ int launch_plain_src(Src src, Out *Aout, int n, int lda, long long batch, int ar
   const bool correct = status_or != 0 && arith == ARITH_FUSED && Aout == nullptr &&
                        n >= kCorrectMinN && n <= kCorrectMaxN;
   const size_t corr_smem = (size_t)n * (n + 1) * sizeof(float2) + 2 * (size_t)n * sizeof(int);
-  // fused, n <= kWarpMaxN, a batch that fills its rounds of a warp per matrix:
-  // no barriers (8192 LLL x n=33 1055 us against 1163 by groups, x n=36 1310
-  // against 1405, 4096 x n=40 899 against 903; reference arithmetic 2219 against
-  // 2211; a part-filled round costs a whole one: 1900 x n=33 344 against 300)
+  // fused, n <= kWarpMaxN: a warp per matrix, without barriers, where the batch
+  // fills its rounds. A part-filled round costs a whole one; groups cost 2% more per
+  // matrix and a tenth of a round for their tail (us, warps | groups: x n=33 1700
+  // 230 | 246, 3500 454 | 462, 8192 (4.5 of 5 rounds) 1055 | 1050; x n=36 4500 (3.7
+  // of 4) 749 | 726; x n=40 3500 (2.9 of 3) 725 | 741, 8192 (6.7 of 7) 1679 | 1654).
+  // Reference arithmetic gains nothing (4096 x n=40 2219 | 2211).
   bool warp_each = false;
   if (n >= kGroupMinN && n <= kWarpMaxN && !correct && arith == ARITH_FUSED) {
     const long long round = 4ll * (long long)((device_smem_optin() + 1024) /
                                               (sub_smem(n, 32) + 1024)) * device_sm_count();
     const long long rounds = (batch + round - 1) / round;
-    warp_each = 100 * batch >= 85 * rounds * round;
+    warp_each = 102 * batch + 10 * round >= 100 * rounds * round;
   }
   if (n >= kGroupMinN && !warp_each) {
     const int threads = group_warps(n) * 32;

@@ -150,7 +150,8 @@ __device__ int lup_fp64_sub(double2 *M, int lds, double *hold, int n, int sub, u
     }
     __syncwarp();
     // trailing update on the m x m block, two entries at a time so that one's
-    // loads overlap the other's arithmetic
+    // loads overlap the other's arithmetic; lanes without an entry read T[-1], a
+    // multiplier, which nobody writes
     const int m = n - 1 - j, mm = m * m;
     double2 *T = M + (j + 1) * lds + j + 1;
     const double2 *L = M + (j + 1) * lds + j, *U = M + j * lds + j + 1;
@@ -163,7 +164,7 @@ __device__ int lup_fp64_sub(double2 *M, int lds, double *hold, int n, int sub, u
       w.next(m);
       const bool on0 = live && e < mm, on1 = live && e + LPM < mm;
       if (e0 + LPM < mm) {  // uniform: no FP64 work for a second half that is empty
-        const int f0 = on0 ? i0 * lds + k0 : 0, f1 = on1 ? i1 * lds + k1 : 0;
+        const int f0 = on0 ? i0 * lds + k0 : -1, f1 = on1 ? i1 * lds + k1 : -1;
         const double2 s0 = T[f0], l0 = L[on0 ? i0 * lds : 0], u0 = U[on0 ? k0 : 0];
         const double2 s1 = T[f1], l1 = L[on1 ? i1 * lds : 0], u1 = U[on1 ? k1 : 0];
         const double2 r0 = cmsub<ARITH>(s0, l0, u0), r1 = cmsub<ARITH>(s1, l1, u1);

@@ -6,11 +6,13 @@ configuration on which the mixed-vs-FP64 target is quoted. A "step" is one
 batched determinant call over the whole batch. The batch is 302 MB, larger than
 the 129 MB L2, so no flush is needed between steps.
 
-Prints ONE JSON line (rank 0). `value` is mixed-precision determinants/s with
-the batch resident in HBM; `e2e` is the same call through the C-ABI with the
-batch copied from pinned host memory each step and the results copied back.
-The plain FP64 kernels, accuracy against the double-double oracle, the
-roofline of the dominant kernel and the CPU baseline ride along in the line.
+Prints ONE JSON line on stdout (rank 0), short enough to survive a cut log.
+`value` is mixed-precision determinants/s with the batch resident in HBM; `e2e`
+is the same call through the C-ABI with the batch copied from pinned host memory
+each step and the results copied back. The plain FP64 kernels, accuracy against
+the double-double oracle, the roofline of the dominant kernel, the CPU baseline
+and the other configurations' rates ride along in the line; everything measured
+goes to stderr as one more JSON line.
 
 `--impl reference` times the reference's CPU Crout path instead: the FP64
 restatement of LUCoreCPU::determinant (the reference is float32-only and its
@@ -883,6 +885,35 @@ def base_line(args, world) -> dict:
             "data": "synthetic (seeded, generated on device)"}
 
 
+# What of a result goes into the printed line; the rest is in the details.
+LINE_KEYS = {
+    "accuracy": ("compared", "max_rel_err", "count_above_1e-10"),
+    "roofline": ("kernel", "bound", "unit", "peak", "achieved", "frac", "traffic",
+                 "kernel_ms_per_launch", "share_of_step"),
+    "e2e": ("value", "unit", "ms_per_step", "h2d_bytes_per_step", "d2h_bytes_per_step",
+            "host_link_copy_gbs", "fraction_of_link"),
+    "e2e_from_coordinates": ("value", "unit", "ms_per_step", "h2d_bytes_per_step",
+                             "d2h_bytes_per_step"),
+    "configs": ("value", "unit", "ms_per_step", "p50_ms", "p99_ms"),
+}
+LINE_DROPS = ("kernel_times_ms", "per_n", "autotune", "serving")
+
+
+def headline(line: dict) -> dict:
+    """The result as it is printed: every key of the benchmark's line, the larger
+    objects cut to the figures that a reader of the line needs."""
+    short = {}
+    for k, v in line.items():
+        if k in LINE_DROPS:
+            continue
+        keep = LINE_KEYS.get(k)
+        if keep and isinstance(v, dict):
+            pick = (lambda d: {q: d[q] for q in keep if d.get(q) is not None})
+            v = {c: pick(d) for c, d in v.items() if d} if k == "configs" else pick(v)
+        short[k] = v
+    return short
+
+
 def run_ours(args):
     world, rank, local = dist_setup(args)
     if args.workload == "mixedn":
@@ -896,7 +927,7 @@ def run_ours(args):
     else:
         r = run_batched(args, world, rank, local, args.workload, full=True)
         if args.workload == "lll24" and not args.no_subconfigs:
-            # compact results of the other configurations, in the same line
+            # results of the other configurations, their rates in the same line
             subs = {
                 "config1_gauss8": run_batched(args, world, rank, local, "gauss8", full=False),
                 "config2_gauss16": run_batched(args, world, rank, local, "gauss16", full=False),
@@ -907,7 +938,8 @@ def run_ours(args):
                 r["configs"] = subs
     if rank == 0 and r is not None:
         line = base_line(args, world) | r
-        print(json.dumps(line), flush=True)
+        print(json.dumps({"details": line}), file=sys.stderr, flush=True)
+        print(json.dumps(headline(line)), flush=True)
 
 
 def workload_config(workload: str, world: int) -> dict:

@@ -5,10 +5,10 @@
 // items are ordered largest n first (longest-processing-time first, so the
 // short small-n items fill the tail), stored in device memory, and consumed
 // by a persistent kernel: each warp takes the next item with one atomicAdd on
-// a device counter and runs the per-n device routine (the register-tiled
-// mixed routine for n in {6, 8, 12, 16, 24, 32}, the generic one otherwise,
-// or the FP64 routines in the plain modes). Shared memory per warp is sized
-// for the largest n of the batch.
+// a device counter and runs the per-n device routine (mixed: the lane-grid path
+// up to n = 16, several matrices at a time, the register-tiled routine for n = 24
+// and 32, the generic one otherwise; or the FP64 routines). Shared memory per warp
+// is sized for the largest n of the pass.
 //
 // A plan (lufqhe_plan_create) fixes the groups and output buffers, chooses the
 // tile sizes and the warps per CTA with an autotuner that times candidate
@@ -487,9 +487,9 @@ GroupedKernel group_kernel_for(int mode, bool correct) {
 }
 
 // One pass of a plan: a grouped kernel over its own work list. A plan runs up
-// to three passes back to back:
+// to four passes back to back:
 //  0. the plan's mode over the groups on the warp-per-matrix path (a mixed
-//     plan's FP32-path groups; a plain plan's groups with n <= 32);
+//     plan's FP32-path groups with n > kSmallMaxN; a plain plan's with n <= 32);
 //  1. (mixed plans) the plain fused kernel over the groups with n <= 32 that
 //     the precision policy sends to FP64;
 //  2. the warp-group kernel over the FP64-route groups with n > 32 (fused

@@ -1,8 +1,11 @@
 // The mixed method's FP32 path for n <= 32, several small matrices per warp.
 //
 // The steps and every rounded operation are those of mixed_core.cuh (the
-// register-tiled path there, and for other sizes the generic one), so results
-// are the same bits; what differs is where the work sits:
+// register-tiled path there, and for other sizes the generic one), so an accepted
+// matrix has the same bits; only the generic rule's ||E||_F is summed in another
+// order (that of a 4 x 8 lane grid), so a matrix within rounding of the acceptance
+// bound may be accepted here and refactorised there, or the reverse. What differs
+// is where the work sits:
 //  * A matrix has GR x GC lanes: 8 for n <= 8, 16 for n <= 16, 32 above, so a
 //    warp factorises 4, 2 or 1 matrices in lockstep. At n = 8 the serial parts
 //    of a factorisation (pivot searches, reciprocals, reductions, the log

@@ -30,7 +30,7 @@
 // Warps take matrices from a work counter rather than a fixed grid stride: a
 // matrix refactorised in FP64 costs many times an accepted one, and a fixed
 // share of the batch per warp would leave the kernel waiting on the warps
-// that drew the most of them. For n >= 24 the refinements and FP64
+// that drew the most of them. At n = 24 and 32 the refinements and FP64
 // refactorisations run after the FP32 pass, in a second kernel on the same
 // stream that has the whole GPU: the FP32 pass saves a matrix whose
 // correction is within theta but beyond what FP32 solves carry (its L\U and
@@ -38,22 +38,23 @@
 // the index of a rejected matrix to the call's pending list; the second
 // kernel deals the list's entries out to its warps at a fixed stride for FP64
 // while the other warps refine the saved matrices, so the FP64 and FP32 pipes
-// work side by side. The other sizes take the lane-grid path (mixed_grid.cuh): for
-// n <= 16, where the FP64 refactorisations are cheap and rare enough that a
-// second launch costs more than it saves, it refines and refactorises in place,
-// and so does the n = 24, 32 variant that reads its batch over the host link
-// (INPLACE); at 17 <= n <= 31 (without a register-tiled kernel) the rejected
-// matrices go to lup_mixed_fallback_kernel. The kernels take their matrices from a source:
-// dense matrices in the reference layout, or lowest-Landau-level orbital
-// matrices built from particle coordinates.
+// work side by side; a third corrects the FP64 factors it listed. For n <= 16, where
+// the FP64 refactorisations are cheap and rare enough that a second launch costs
+// more than it saves, the FP32 pass refines and refactorises in place, and so does
+// the n = 24, 32 variant that reads its batch over the host link
+// (lup_mixed_tile_kernel); at 17 <= n <= 31 without a register-tiled rule the
+// rejected matrices go to lup_mixed_fallback_kernel, but for small batches of
+// n <= 23. The FP32 pass of every n <= 32 is the lane-grid kernel
+// (mixed_grid.cuh). The kernels take their matrices from a source: dense matrices in
+// the reference layout, or matrices built from coordinates or permutations.
 //
 // Every call owns its state: the work counter, the pending list (room for the
-// whole batch) and the saved matrices sit in one block from the library's
-// stream-ordered pool whose head is zeroed on the call's stream before the
-// first kernel. Nothing is shared between calls, so any number of them may be
-// in flight on any streams, and a captured call replays on its own memory. A
-// call whose batch fits in two strides of its grid needs no counter (warps
-// take matrices at a fixed stride) and takes no block.
+// whole batch), the saved matrices and the factor list sit in one block from the
+// library's stream-ordered pool whose head is zeroed on the call's stream before
+// the first kernel. Nothing is shared between calls, so any number of them may be
+// in flight on any streams, and a captured call replays on its own memory. A call
+// whose batch fits in two strides of its grid needs no counter (warps take
+// matrices at a fixed stride) and, without a list, takes no block.
 
 #pragma once
 
@@ -100,7 +101,7 @@ struct CallHead {
 constexpr size_t kHeadBytes = 256;
 
 // A warp's first matrix is its own index in the grid; later ones come from the
-// call's counter (after the grid's warps), or, for a call without one (a batch
+// call's counter (after the grid's warps), or, for a call that needs none (a batch
 // within two strides of the grid), at the grid's stride. Small batches, where
 // most warps take one matrix, then make no same-address atomics at the start
 // (n=8, 4096 matrices: 31.0 -> 28.9 us).
@@ -117,7 +118,6 @@ __device__ __forceinline__ long long claim_matrix(CallHead *head, int lane, long
 // flag LUFQHE_ST_FP64) rather than a rejection (LUFQHE_ST_FALLBACK).
 constexpr unsigned int kPendRouted = 0x80000000u;
 
-constexpr int kDeferMinN = 24;
 // Matrices per SM up to which a batch of 17 <= n <= 23 refactorises in place: one
 // launch and no state block (64 Gaussian matrices of n = 20: 39.0 us with a second
 // kernel, 35.5 in place; 500 LLL 147, 136; 1000 LLL 160, 150). Beyond that the
@@ -211,6 +211,9 @@ __device__ __noinline__ bool save_refine(CallHead *head, unsigned char *buf, lon
   return true;
 }
 
+// The FP32 pass above n = 32, where the precision policy takes it (a share below 1
+// under LUFQHE_OPT_FP64_SHARE): a warp per matrix in shared memory, the rejected
+// matrices to the call's pending list.
 template <class Src>
 __global__ void __launch_bounds__(kMaxWarpsMixed * 32)
     lup_mixed_kernel(Src src, int n, long long batch,
@@ -253,11 +256,8 @@ __global__ void __launch_bounds__(kMaxWarpsMixed * 32)
     float2 corr;
     if (mixed_factor(S, n, lane, theta2, prod, exp_sum, corr, par))
       out.push(lane, b, prod, exp_sum, corr, par, logabs, phase, parity, status);
-    else if (pend)
-      defer_fp64(head, pend, b, lane, false);
     else
-      fallback_fp64_src(src, b, n, M, lds, S.hold, lane, b, logabs, phase, parity, status,
-                        LUFQHE_ST_FALLBACK, &cs);
+      defer_fp64(head, pend, b, lane, false);
   }
   out.flush(lane, logabs, phase, parity, status);
 }
@@ -573,8 +573,8 @@ __global__ void __launch_bounds__(kFacCorrectWarps * 32, 8)
   }
 }
 
-// The FP64 pass of the generic mixed kernel (n >= 24 without a register-tiled
-// kernel): one CTA per SM; its warps refactorise the pending list's matrices
+// The FP64 pass of the sizes without a register-tiled kernel (17 <= n <= 31, and
+// above 32): one CTA per SM; its warps refactorise the pending list's matrices
 // (reference pivot rule, fused arithmetic, status flag LUFQHE_ST_FALLBACK, or
 // LUFQHE_ST_FP64 for the routed share). Every factorisation of one n costs the
 // same, so the entries are dealt out at a fixed stride: entry j goes to warp
@@ -1060,14 +1060,9 @@ int launch_mixed_src(Src src, int n, long long batch, double *logabs, double *ph
   long long cap = (long long)device_sm_count() * per_sm;
   int grid = (int)(want < cap ? want : cap);
   const float theta2 = g_mixed_theta * g_mixed_theta;
-  // n >= 24: rejected matrices go to the FP64 pass through the call's list
-  const bool two_pass = n >= kDeferMinN;
-  const bool counter = needs_counter(batch, (long long)grid * warps);
   CallState cs;
-  if (two_pass || counter) {
-    rc = cs.acquire(two_pass ? (size_t)batch : 0, 0, 0, stream);
-    if (rc) return cs.release(stream, rc);
-  }
+  rc = cs.acquire((size_t)batch, 0, 0, stream);
+  if (rc) return cs.release(stream, rc);
   {
     KernelTimer timer("lup_mixed_kernel", n, stream);
     kern<<<grid, warps * 32, smem, stream>>>(src, n, batch, theta2, fp64_share_64k(n),
@@ -1075,7 +1070,7 @@ int launch_mixed_src(Src src, int n, long long batch, double *logabs, double *ph
     timer.stop();
   }
   rc = check_cuda(cudaGetLastError(), "lup_mixed_kernel launch");
-  if (!rc && two_pass)
+  if (!rc)
     rc = launch_fallback(src, n, cs.head, cs.pend, batch, logabs, phase, parity, status, stream);
   return cs.release(stream, rc);
 }

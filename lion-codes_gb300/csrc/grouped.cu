@@ -265,7 +265,11 @@ __global__ void __launch_bounds__(kMaxWarpsMixed * 32, 1)
 // warp taking an item's matrices several at a time (the batched call's path and
 // bits, on its grid of the size). nm, the pass's largest n, sizes a warp's
 // shared memory.
-template <int NP, int NC>
+// ROUTED: some item has a share routed to FP64; such an item's units are its
+// matrices that are not, and the ones in between go to FP64 on the way. (A kernel
+// of its own: with one for both, plans of a few hundred small matrices took 2 us,
+// 4%, longer.)
+template <int NP, int NC, bool ROUTED>
 __device__ void small_item(const WorkItem &w, unsigned char *base, int lane, float theta2,
                            bool refine, DeferredOut &out, double *logabs, double *phase,
                            int8_t *parity, int32_t *status) {
@@ -276,39 +280,43 @@ __device__ void small_item(const WorkItem &w, unsigned char *base, int lane, flo
   const DenseSource src{w.A, w.lda};
   const int n = NC ? NC : w.n;
   double2 *M = reinterpret_cast<double2 *>(HLw);
-  for (int j = 0; j < w.count;) {
-    // the unit: G consecutive matrices, or, where a share is routed to FP64, the
-    // next G that are not (the ones in between go to FP64 on the way)
-    int cnt = 0, mine = 0;
-    if (!w.share64k) {
-      cnt = min(Gd::G, w.count - j);
-      mine = j + lane / Gd::LPM;
-      j += cnt;
-    }
-    for (; w.share64k && cnt < Gd::G && j < w.count; ++j) {
-      if (route_fp64_entry(src.first(w.first + j, n), w.share64k)) {
-        grid_refactor_call<NP>(src, w.first + j, n, HLw, Fw, Iw, lane, w.out + j, logabs, phase,
-                               parity, status, LUFQHE_ST_FP64);
-      } else {
-        if (cnt == lane / Gd::LPM) mine = j;
-        ++cnt;
-      }
-    }
-    if (cnt == 0) break;
-    auto at = [&](int q) { return __shfl_sync(kFull, mine, q * Gd::LPM); };
-    __syncwarp();
-    if (!w.share64k)
-      load_rows(src, w.first + at(0), cnt * n, n, M, Gd::LDH, NP, lane);
-    else
-      for (int q = 0; q < cnt; ++q)
-        load_rows(src, w.first + at(q), n, n, M + q * Gd::kHL, Gd::LDH, NP, lane);
-    __syncwarp();
+  auto unit = [&](int cnt, auto at) {
     grid_unit<NP, Gd::LPM, NC, true, true>(
         src, w.first, w.out, cnt, n, HLw, Fw, Iw, lane, theta2, 0u, refine, at,
         [](long long, bool, bool, const CFF &, int, int) {}, out, logabs, phase, parity, status);
+  };
+  if constexpr (!ROUTED) {
+    for (int j = 0; j < w.count; j += Gd::G) {
+      const int cnt = min(Gd::G, w.count - j);
+      __syncwarp();
+      load_rows(src, w.first + j, cnt * n, n, M, Gd::LDH, NP, lane);
+      __syncwarp();
+      unit(cnt, [j](int q) { return j + q; });
+    }
+  } else {
+    for (int j = 0; j < w.count;) {
+      int cnt = 0, mine = 0;
+      for (; cnt < Gd::G && j < w.count; ++j) {
+        if (route_fp64_entry(src.first(w.first + j, n), w.share64k)) {
+          grid_refactor_call<NP>(src, w.first + j, n, HLw, Fw, Iw, lane, w.out + j, logabs, phase,
+                                 parity, status, LUFQHE_ST_FP64);
+        } else {
+          if (cnt == lane / Gd::LPM) mine = j;
+          ++cnt;
+        }
+      }
+      if (cnt == 0) break;
+      auto at = [mine](int q) { return __shfl_sync(kFull, mine, q * Gd::LPM); };
+      __syncwarp();
+      for (int q = 0; q < cnt; ++q)
+        load_rows(src, w.first + at(q), n, n, M + q * Gd::kHL, Gd::LDH, NP, lane);
+      __syncwarp();
+      unit(cnt, at);
+    }
   }
 }
 
+template <bool ROUTED>
 __global__ void __launch_bounds__(kMaxWarpsMixed * 32, 2)
     grouped_small_kernel(const WorkItem *__restrict__ items, int nitems, unsigned int *counter,
                          int nm, int nf, float theta2, int refine, double *__restrict__ logabs,
@@ -328,15 +336,15 @@ __global__ void __launch_bounds__(kMaxWarpsMixed * 32, 2)
     const WorkItem w = items[it];
     const bool rf = refine != 0;
     switch (w.n) {
-      case 6: small_item<8, 6>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
-      case 8: small_item<8, 8>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
-      case 12: small_item<12, 12>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
-      case 16: small_item<16, 16>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
+      case 6: small_item<8, 6, ROUTED>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
+      case 8: small_item<8, 8, ROUTED>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
+      case 12: small_item<12, 12, ROUTED>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
+      case 16: small_item<16, 16, ROUTED>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
       default:
         switch (small_np(w.n)) {
-          case 8: small_item<8, 0>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
-          case 12: small_item<12, 0>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
-          default: small_item<16, 0>(w, base, lane, theta2, rf, out, logabs, phase, parity, status);
+          case 8: small_item<8, 0, ROUTED>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
+          case 12: small_item<12, 0, ROUTED>(w, base, lane, theta2, rf, out, logabs, phase, parity, status); break;
+          default: small_item<16, 0, ROUTED>(w, base, lane, theta2, rf, out, logabs, phase, parity, status);
         }
     }
   }
@@ -346,12 +354,14 @@ __global__ void __launch_bounds__(kMaxWarpsMixed * 32, 2)
 using GroupedKernel = void (*)(const WorkItem *, int, unsigned int *, int, int, float, int,
                                double *, double *, int8_t *, int32_t *, PlanAux);
 
-GroupedKernel kernel_for(int mode, bool small = false) {
+// routed: the small pass has a group with a share routed to FP64
+GroupedKernel kernel_for(int mode, bool small = false, bool routed = false) {
   switch (mode) {
     case LUFQHE_MODE_PLAIN_FP64: return grouped_kernel<LUFQHE_MODE_PLAIN_FP64>;
     case LUFQHE_MODE_PLAIN_FP64_FUSED: return grouped_kernel<LUFQHE_MODE_PLAIN_FP64_FUSED>;
     default:
-      return small ? grouped_small_kernel : grouped_kernel<LUFQHE_MODE_MIXED>;
+      if (small) return routed ? grouped_small_kernel<true> : grouped_small_kernel<false>;
+      return grouped_kernel<LUFQHE_MODE_MIXED>;
   }
 }
 
@@ -503,6 +513,7 @@ GroupedKernel group_kernel_for(int mode, bool correct) {
 struct Launch {
   int mode = LUFQHE_MODE_MIXED;
   int nm = 0, nf = 1;  // warp_layout of the pass
+  bool routed = false;  // a group with a share routed to FP64
   int warps = 4;
   int ctas = 0;        // grid size
   size_t smem = 0;
@@ -626,10 +637,12 @@ int configure_pass(lufqhe_plan_s *p, int pass, int warps) {
                                                                     : p->mode;
   L.nm = 0;
   L.nf = 0;
+  L.routed = false;
   for (size_t g = 0; g < p->groups.size(); ++g) {
     const lufqhe_group_t &G = p->groups[g];
     if (G.count == 0 || pass_of(p, g) != pass) continue;
     L.nf = std::max(L.nf, G.n);
+    L.routed |= p->share[g] != 0;
     if (L.mode == LUFQHE_MODE_MIXED) L.nm = std::max(L.nm, G.n);
     // a mixed plan's FP64 route with corrected sizes: the correction's
     // scratch (the FP32 path's F and ints) in the layout
@@ -670,7 +683,7 @@ int configure_pass(lufqhe_plan_s *p, int pass, int warps) {
     L.ctas = device_sm_count() * per_sm;
     return LUFQHE_SUCCESS;
   }
-  GroupedKernel k = kernel_for(L.mode, pass == 3);
+  GroupedKernel k = kernel_for(L.mode, pass == 3, L.routed);
   const size_t per_warp = pass == 3 ? small_warp_bytes(L.nm) : warp_layout(L.nm, L.nf).total;
   const size_t optin = device_smem_optin();
   int w = std::min<int>(warps, (int)(optin / per_warp));
@@ -717,7 +730,7 @@ int launch_once(lufqhe_plan_s *p, cudaStream_t s) {
     const Launch &L = p->launch[pass];
     if (L.nitems == 0 || L.ctas == 0) continue;
     GroupedKernel k =
-        pass == 2 ? group_kernel_for(L.mode, L.nm > 0) : kernel_for(L.mode, pass == 3);
+        pass == 2 ? group_kernel_for(L.mode, L.nm > 0) : kernel_for(L.mode, pass == 3, L.routed);
     // a warp-group CTA takes one item at a time
     const long long want = pass == 2 ? L.nitems : (L.nitems + L.warps - 1) / L.warps;
     const int grid = (int)std::min<long long>(L.ctas, want);

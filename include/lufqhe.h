@@ -416,30 +416,32 @@ long long lufqhe_read_matrices_f32(const char *path, int n, long long first, lon
  * 0.1; 0 sends every matrix to the FP64 path, +inf disables the fallback
  * except for zero or non-finite FP32 pivots). */
 #define LUFQHE_OPT_MIXED_THRESHOLD 1
-/* Warps per CTA of the register-tiled mixed kernels (n in {6,8,12,16,24,32});
- * 0 = library default. */
+/* Warps per CTA (0..8) of the batched mixed kernels of the register-tiled sizes
+ * (n in {6,8,12,16,24,32}) but the correction pass; values above what a kernel is
+ * built for (3 warps at n = 24, 4 elsewhere) and 0 mean the library's default. */
 #define LUFQHE_OPT_TILE_WARPS 2
 /* Fraction (0..1) of the matrices the batched mixed mode sends straight to the
  * FP64 routine, chosen by a hash of each matrix's first entry (so a matrix
- * takes the same path wherever it sits); the FP64 pipe then works beside the
- * FP32 pipes. A negative value restores the per-n default. */
+ * takes the same path wherever it sits); the FP32 path does not look at them. A
+ * negative value restores the per-n default. */
 #define LUFQHE_OPT_FP64_SHARE 3
 /* Input bytes per chunk of lufqhe_batch_lup_det_host, in MiB (1..1024; default
  * 32). */
 #define LUFQHE_OPT_HOST_CHUNK_MB 4
-/* Mixed mode, n = 24 and 32: 1 (default) refines the back substitution of the
- * matrices whose correction the FP32 solves cannot carry to 1e-10 but whose
- * ||E||_F is within the threshold, in a pass of its own, before sending the
- * rest to FP64; 0 sends them all to FP64. */
+/* Mixed mode, n in {6,8,12,16,24,32}: 1 (default) refines the back substitution of
+ * the matrices whose correction the FP32 solves cannot carry to 1e-10 but whose
+ * ||E||_F is within the threshold (at n = 24 and 32 in a pass of its own) before
+ * sending the rest to FP64; 0 sends them all to FP64. */
 #define LUFQHE_OPT_MIXED_REFINE 5
 /* 1: the batched entry points record a CUDA event pair around every kernel
  * they launch, on the launching stream, for lufqhe_kernel_times (not while
  * the stream is being captured); 0 (default): no events. */
 #define LUFQHE_OPT_KERNEL_TIMING 6
-/* 1 (default): the plain FP64 warp kernel and the n >= 24 mixed FP32 pass
- * stage each complex128 matrix from device memory into shared memory with
- * the copy engine's bulk copies (one per row, completing on an mbarrier) and
- * prefetch the next matrix into L2; 0: per-lane vector loads. Same bits. */
+/* 1 (default): the plain FP64 kernels with a warp or less per matrix and the mixed
+ * FP32 pass of n <= 32 stage complex128 matrices from device memory into shared
+ * memory with the copy engine's bulk copies (one per row, completing on an
+ * mbarrier) and prefetch the next ones into L2; 0: per-lane vector loads. Same
+ * bits. */
 #define LUFQHE_OPT_BULK_LOADS 7
 /* Servers created while this is 1 keep each walker matrix's FP64
  * L\U factors and take a move's determinant ratio from an O(n^2) solve
@@ -484,10 +486,15 @@ int lufqhe_kernel_times(char *json, size_t len);
 
 /* ---- misc ---- */
 /* Bytes of device memory a lufqhe_batch_lup_det call of this n, batch and mode
- * takes, stream-ordered, from the library's own memory pool while it runs
- * (mixed mode at n = 24 and 32: the matrices saved for the refinement of the
- * back substitution, room for a quarter of the batch; 0 otherwise). The pool
- * keeps freed blocks for the next call. */
+ * takes at most, stream-ordered, from the library's own memory pool while it runs,
+ * but for the factor list of n = 24 and 32. Mixed mode, under the options as they
+ * are: 256 bytes (the call's counters); for 17 <= n, and for smaller n with a
+ * routed share, a list of 4 bytes per matrix (small batches of n <= 23 take none);
+ * at n = 24 and 32 the matrices saved for the refinement of the back substitution,
+ * room for a quarter of the batch. The factor list, not counted, has room for a
+ * quarter of the batch as well (16 n^2 + 4 n + 32 bytes an entry, and 16 n^2 more
+ * for complex64 or built matrices). 0 for the plain modes and where the policy
+ * sends every matrix to FP64. The pool keeps freed blocks for the next call. */
 size_t lufqhe_workspace_bytes(int n, long long batch, int mode);
 /* Return the library pool's unused device memory to the driver, on every
  * device the library has used. Blocks still held by work in flight stay
